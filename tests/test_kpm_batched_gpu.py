@@ -58,3 +58,40 @@ def test_device_status_clean(dev):
     from vbcsr_b200 import _capi
 
     assert _capi.device_status(clear=True) == 0
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_segment_sums_over_chunk_edges(dev, precision):
+    """Per-segment sums at the edges of the 512-row chunks: an empty segment,
+    exactly one chunk, a single row, a whole number of chunks and a
+    remainder.  The recurrence itself does not depend on the segments, so a
+    segment's moment is the plain one restricted to its rows (FP64 sums
+    1e-12 of mu_0; FP32 vectors 1e-5, one rounding of 6e-8 per step and
+    element)."""
+    import ctypes as C
+
+    import torch
+
+    from vbcsr_b200 import _capi
+
+    H, _ = W.tmd_lattice(30, seed=8)
+    seg = np.array([0, 0, 512, 513, 1537, H.n], np.int32)
+    R, M = 16, 9
+    V = np.where(np.random.default_rng(2).random((H.N, R)) < 0.5, -1.0, 1.0)
+    i, j = W.scalar_coords(H)
+    A = torch.sparse_coo_tensor(np.stack([i, j]), H.values, (H.N, H.N)).to_sparse_csr()
+    Vt = torch.from_numpy(V)
+    ts = [Vt, A @ Vt]
+    while len(ts) < M:
+        ts.append(2 * (A @ ts[-1]) - ts[-2])
+    so = H.scalar_offsets()[seg]
+    ref = np.array([[float((Vt * t)[a:b].sum()) for t in ts] for a, b in zip(so[:-1], so[1:])])
+    dm = _capi.DeviceMatrix.create(H.block_sizes, H.row_ptr, H.col_ind, H.values)
+    Vd = Vt.cuda().contiguous()
+    mu = torch.full((len(seg) - 1, M), -1.0, dtype=torch.float64, device="cuda")
+    for _ in range(2):  # the second call replays the graph (its counters were reset)
+        _capi.call("vbg_kpm_moments_batched", dm.h, len(seg) - 1, seg.ctypes.data_as(C.POINTER(C.c_int)), R, R,
+                   C.c_void_p(Vd.data_ptr()), M, precision, 0, 1, C.c_void_p(mu.data_ptr()), None)
+        torch.cuda.synchronize()
+        err = np.abs(mu.cpu().numpy() - ref).max(axis=1) / np.maximum(ref[:, 0], 1.0)
+        assert err.max() < (1e-5 if precision else 1e-12), err

@@ -309,8 +309,11 @@ struct vbg_matrix {
   vbg::DevBuf partials, counter;
   // KPM workspace and graph cache
   vbg::DevBuf kpm_ws, kpm_dots;
-  // batched KPM: per-row dots, segment boundaries (block rows, scalar rows)
-  vbg::DevBuf kpm_rowdots, kpm_seg, kpm_segscal;
+  // batched KPM: per-row dots; the segments' row chunks ({segment, first
+  // row, end row, first chunk of the segment}), each segment's chunk range,
+  // the chunks' partial sums and a done counter per segment
+  vbg::DevBuf kpm_rowdots, kpm_chunks, kpm_segchunk, kpm_segpart, kpm_segcnt;
+  int kpm_nchunks = 0;
   std::vector<int> kpm_seg_host;
   std::map<std::tuple<int, int, const void*, int, int, int, double*>, std::unique_ptr<vbg::GraphEntry>> graphs;
   cudaStream_t graph_stream = nullptr;
@@ -342,7 +345,7 @@ struct vbg_matrix {
     for (vbg::DevBuf* b : {&row_ptr, &col_ind, &bsz, &scal_off, &blk_off, &diag_slot, &row_perm, &slot_meta, &srow, &scol, &csc_meta, &csc_boff, &vals,
                            &vals32, &valsK, &valsK32, &koff, &koff32, &spans, &span_koff32, &row_sptr, &csc_ptr,
                            &csc_slot, &csc_row, &csc_perm, &partials, &counter, &kpm_ws, &kpm_dots, &kpm_rowdots,
-                           &kpm_seg, &kpm_segscal})
+                           &kpm_chunks, &kpm_segchunk, &kpm_segpart, &kpm_segcnt})
       b->release_synced();
   }
 };
