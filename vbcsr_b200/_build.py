@@ -24,6 +24,7 @@ LIB = HERE / "libvbcsr_b200.so"
 CUDA_SOURCES = [
     "vbg_matrix.cu",
     "vbg_apply.cu",
+    "vbg_mma.cu",
     "vbg_vec.cu",
     "vbg_algebra.cu",
     "vbg_spgemm.cu",

@@ -26,50 +26,12 @@
 #include <type_traits>
 
 #include "vbg_internal.cuh"
+#include "vbg_args.cuh"
 
 namespace vbg {
 
 constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
-
-struct ApplyArgs {
-  int n_rows;                // output block rows
-  const int* order;          // visiting order of output rows (nullptr = natural)
-  const int* ptr;            // entry range per output row (row_ptr or csc_ptr)
-  const int* ent_slot;       // adjoint: slot of each entry (forward: entry == slot)
-  const int* ent_src;        // source block of each entry (col_ind or csc_row)
-  const int* bsz;
-  const int64_t* scal_off;
-  const int64_t* blk_off;
-  const int2* slot_meta;     // forward: per slot {first X row of the block column, rows << 8 | cols}
-  const int64_t* koff;       // pipelined kernel: per-slot offsets of the kernel-layout values
-  const int4* spans;         // pipelined kernel: spans, FP32 layout offsets, each block row's span range
-  const int64_t* span_koff32;
-  const int* row_sptr;
-  int ld;                    // leading dimension of X/Y in elements (1 = vector)
-  // epilogue  Y = alpha * (A X) + beta * X + gamma * Xprev
-  double alpha, beta, gamma;
-  const void* X;
-  const void* Xprev;
-  void* Y;
-  const void* dotw;          // dot partner for dots[0] (nullptr -> X)
-  void* acc;                 // acc += acc_coef * Y (nullptr -> none)
-  double cre, cim;
-  int want_dots;
-  double* row_dots;          // with want_dots: per block row (d0, d1) here instead of the grid reduction
-  double* partials;
-  unsigned* counter;
-  double* dots_out;
-  int max_ctas;              // CTAs `partials` has room for (0: max_total_ctas())
-  // vector apply: ranges each CTA prefetches its share of into L2 at start
-  // (16-byte aligned; set when the whole working set fits L2)
-  int npf;
-  const void* pf_ptr[4];
-  long long pf_bytes[4];
-  // scalar-row vector apply: per scalar row {first slot, count << 8 | row in block}, scalar rows
-  const int2* srow;
-  int64_t n_scal;
-};
 
 template <typename T> struct VT;
 template <> struct VT<double> { using raw = double2; static constexpr int E = 2; };
@@ -94,15 +56,6 @@ __device__ __forceinline__ void store_vec(T* base, int64_t vidx, const Vec<T>& v
   memcpy(&r, &v, sizeof(r));
   reinterpret_cast<typename VT<T>::raw*>(base)[vidx] = r;
 }
-
-__device__ __forceinline__ double shfl_xor_s(double v, int off) { return __shfl_xor_sync(0xffffffffu, v, off); }
-__device__ __forceinline__ float shfl_xor_s(float v, int off) { return __shfl_xor_sync(0xffffffffu, v, off); }
-__device__ __forceinline__ cplx shfl_xor_s(cplx v, int off) {
-  return {__shfl_xor_sync(0xffffffffu, v.re, off), __shfl_xor_sync(0xffffffffu, v.im, off)};
-}
-__device__ __forceinline__ double add_s(double a, double b) { return a + b; }
-__device__ __forceinline__ float add_s(float a, float b) { return a + b; }
-__device__ __forceinline__ cplx add_s(cplx a, cplx b) { return {a.re + b.re, a.im + b.im}; }
 
 // Epilogue for one output element.
 template <typename T>
@@ -281,9 +234,9 @@ __device__ __forceinline__ bool dispatch_vec_row_meta(const ApplyArgs& a, const 
 // lanes [grp*LPR, grp*LPR + LPR) cover 16-byte vectors of the padded X row;
 // the G lane groups take every G-th block of the row and are summed by
 // butterfly shuffles at the end.  RM output rows per pass (R <= 8 exact).
-template <typename T, int RM, bool ADJ>
+template <typename T, int RM>
 __device__ __forceinline__ void mv_rows(const ApplyArgs& a, const T* __restrict__ vals, int row, int lane, int lpr,
-                                        int G, int o0, int rcount, int rfull, double& d0, double& d1) {
+                                        int G, int o0, int rcount, double& d0, double& d1) {
   constexpr int E = VT<T>::E;
   const int grp = lane / lpr;
   const int vl = lane - grp * lpr;
@@ -301,17 +254,15 @@ __device__ __forceinline__ void mv_rows(const ApplyArgs& a, const T* __restrict_
     if (valid) {
       for (int e = e0 + grp; e < e1; e += G) {
         const int src = a.ent_src[e];
-        const int s = ADJ ? a.ent_slot[e] : e;
         const int inner = a.bsz[src];
         const int64_t xrow0 = a.scal_off[src];
-        const T* ab = vals + a.blk_off[s];
+        const T* ab = vals + a.blk_off[e];
         for (int q = 0; q < inner; ++q) {
           const Vec<T> xv = load_vec(X, (xrow0 + q) * nvec + vi);
 #pragma unroll
           for (int o = 0; o < RM; ++o) {
             if (o < rcount) {
-              T av = ADJ ? ab[(int64_t)q * rfull + o0 + o] : ab[(int64_t)(o0 + o) * inner + q];
-              if (ADJ) av = conj_s(av);
+              const T av = ab[(int64_t)(o0 + o) * inner + q];
 #pragma unroll
               for (int u = 0; u < E; ++u) acc[o].v[u] = fma_s(av, xv.v[u], acc[o].v[u]);
             }
@@ -380,81 +331,6 @@ __device__ __forceinline__ void dispatch_vec_row(const ApplyArgs& a, const T* __
   }
 }
 
-// Fixed-order two-value reduction across the grid: per-CTA partials, then
-// the last CTA to finish sums them in a fixed tree and resets the counter.
-// Blocks have at most 1024 threads.
-__device__ void grid_reduce2(double d0, double d1, double* partials, unsigned* counter, double* out, int part_base,
-                             int total) {
-  __shared__ double red[32][2];
-  __shared__ bool is_last;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    d0 += __shfl_xor_sync(0xffffffffu, d0, off);
-    d1 += __shfl_xor_sync(0xffffffffu, d1, off);
-  }
-  if (lane == 0) {
-    red[warp][0] = d0;
-    red[warp][1] = d1;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s0 = 0.0, s1 = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      s0 += red[w][0];
-      s1 += red[w][1];
-    }
-    partials[2 * (part_base + blockIdx.x)] = s0;
-    partials[2 * (part_base + blockIdx.x) + 1] = s1;
-    __threadfence();
-    const unsigned prev = atomicAdd(counter, 1u);
-    is_last = (prev == (unsigned)total - 1);
-  }
-  __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  double s0 = 0.0, s1 = 0.0;
-  for (int b = threadIdx.x; b < total; b += blockDim.x) {
-    s0 += __ldcg(partials + 2 * b);
-    s1 += __ldcg(partials + 2 * b + 1);
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    s0 += __shfl_xor_sync(0xffffffffu, s0, off);
-    s1 += __shfl_xor_sync(0xffffffffu, s1, off);
-  }
-  __syncthreads();
-  if (lane == 0) {
-    red[warp][0] = s0;
-    red[warp][1] = s1;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t0 = 0.0, t1 = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      t0 += red[w][0];
-      t1 += red[w][1];
-    }
-    out[0] = t0;
-    out[1] = t1;
-    *counter = 0u;
-  }
-}
-
-// Per-row dot output (batched recurrences): sums this row's lane partials
-// over the warp and writes them; the caller's accumulators are untouched.
-__device__ __forceinline__ void write_row_dots(double* row_dots, int row, double r0, double r1) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    r0 += __shfl_xor_sync(0xffffffffu, r0, off);
-    r1 += __shfl_xor_sync(0xffffffffu, r1, off);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    row_dots[2 * row] = r0;
-    row_dots[2 * row + 1] = r1;
-  }
-}
-
 // This CTA's share of [p, p + bytes) prefetched into L2 by bulk prefetches
 // (16-byte units, 64 KiB per instruction; a tail under 16 bytes is left to
 // the loads).  p is 16-byte aligned.
@@ -494,9 +370,10 @@ __global__ void __launch_bounds__(kThreads) apply_vec_kernel(ApplyArgs a, const 
   if (a.want_dots) grid_reduce2(d0, d1, a.partials, a.counter, a.dots_out, part_base, total);
 }
 
-// Multivectors: one launch per block-size class; rows [w0, w1) of the
-// class-ordered row list all have block size R (R == 0: any size > 8).
-template <typename T, int R, bool ADJ>
+// FP32 multivectors the staged applies do not take: one launch per block-size
+// class; rows [w0, w1) of the class-ordered row list all have block size R
+// (R == 0: any size > 8).  FP64 and complex values run on vbg_mma.cu instead.
+template <typename T, int R>
 __global__ void __launch_bounds__(kThreads) apply_mv_kernel(ApplyArgs a, const T* __restrict__ vals, int w0, int w1,
                                                             int lpr, int G, int part_base, int total) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -505,11 +382,11 @@ __global__ void __launch_bounds__(kThreads) apply_mv_kernel(ApplyArgs a, const T
     const int row = a.order[w];
     double r0 = 0.0, r1 = 0.0;
     if constexpr (R > 0) {
-      mv_rows<T, R, ADJ>(a, vals, row, lane, lpr, G, 0, R, R, r0, r1);
+      mv_rows<T, R>(a, vals, row, lane, lpr, G, 0, R, r0, r1);
     } else {
       const int r = a.bsz[row];
       for (int o0 = 0; o0 < r; o0 += 8)
-        mv_rows<T, 8, ADJ>(a, vals, row, lane, lpr, G, o0, min(8, r - o0), r, r0, r1);
+        mv_rows<T, 8>(a, vals, row, lane, lpr, G, o0, min(8, r - o0), r0, r1);
     }
     if (a.want_dots) {
       if (a.row_dots) {
@@ -583,34 +460,19 @@ static int vec_max_grid() {
   return cached[dev];
 }
 
-template <typename T, int R, bool ADJ>
+template <typename T, int R>
 static int mv_max_grid() {
   static int cached[kMaxDevices] = {};
   const int dev = current_device();
   if (!cached[dev]) {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, apply_mv_kernel<T, R, ADJ>, kThreads, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, apply_mv_kernel<T, R>, kThreads, 0) !=
             cudaSuccess ||
         per_sm < 1)
       per_sm = 1;
     cached[dev] = per_sm * sm_count();
   }
   return cached[dev];
-}
-
-// Largest number of CTAs one apply (all class launches together) can use.
-static int max_total_ctas() { return sm_count() * 8 * 10; }
-
-// A launch that reduces its dots through `partials` must fit them: `total`
-// CTAs of this apply against the room the caller gave (a.max_ctas), else the
-// library's scratch (max_total_ctas()).
-static int check_dot_ctas(const ApplyArgs& a, int total) {
-  if (!a.want_dots || a.row_dots) return 0;
-  const int cap = a.max_ctas > 0 ? a.max_ctas : max_total_ctas();
-  if (total <= cap) return 0;
-  return fail(a.max_ctas > 0 ? VBG_E_ARG : VBG_E_STATE,
-              "this launch needs " + std::to_string(total) + " CTA partial sums; the dot scratch holds " +
-                  std::to_string(cap));
 }
 
 // Working sets up to this size are prefetched into L2 by the vector apply.
@@ -865,32 +727,32 @@ static int launch_vec_t(const vbg_matrix* m, const ApplyArgs& a0, const T* vals,
   return 0;
 }
 
-template <typename T, int R, bool ADJ>
+template <typename T, int R>
 static int launch_mv_class(const ApplyArgs& a, const T* vals, int w0, int w1, int lpr, int G, int grid, int base,
                            int total, cudaStream_t s) {
-  apply_mv_kernel<T, R, ADJ><<<grid, kThreads, 0, s>>>(a, vals, w0, w1, lpr, G, base, total);
+  apply_mv_kernel<T, R><<<grid, kThreads, 0, s>>>(a, vals, w0, w1, lpr, G, base, total);
   VBG_CUDA(cudaGetLastError());
   return 0;
 }
 
-template <typename T, bool ADJ>
+template <typename T>
 static int mv_class_grid(int r, int rows) {
   int cap;
   switch (r) {
-    case 1: cap = mv_max_grid<T, 1, ADJ>(); break;
-    case 2: cap = mv_max_grid<T, 2, ADJ>(); break;
-    case 3: cap = mv_max_grid<T, 3, ADJ>(); break;
-    case 4: cap = mv_max_grid<T, 4, ADJ>(); break;
-    case 5: cap = mv_max_grid<T, 5, ADJ>(); break;
-    case 6: cap = mv_max_grid<T, 6, ADJ>(); break;
-    case 7: cap = mv_max_grid<T, 7, ADJ>(); break;
-    case 8: cap = mv_max_grid<T, 8, ADJ>(); break;
-    default: cap = mv_max_grid<T, 0, ADJ>(); break;
+    case 1: cap = mv_max_grid<T, 1>(); break;
+    case 2: cap = mv_max_grid<T, 2>(); break;
+    case 3: cap = mv_max_grid<T, 3>(); break;
+    case 4: cap = mv_max_grid<T, 4>(); break;
+    case 5: cap = mv_max_grid<T, 5>(); break;
+    case 6: cap = mv_max_grid<T, 6>(); break;
+    case 7: cap = mv_max_grid<T, 7>(); break;
+    case 8: cap = mv_max_grid<T, 8>(); break;
+    default: cap = mv_max_grid<T, 0>(); break;
   }
   return std::max(1, std::min((rows + kWarps - 1) / kWarps, cap));
 }
 
-template <typename T, bool ADJ>
+template <typename T>
 static int launch_mv_t(const vbg_matrix* m, const ApplyArgs& a, const T* vals, cudaStream_t s) {
   const int nvec = a.ld / VT<T>::E;
   int lpr = nvec >= 32 ? 32 : nvec;
@@ -908,7 +770,7 @@ static int launch_mv_t(const vbg_matrix* m, const ApplyArgs& a, const T* vals, c
   std::vector<int> grids;
   int total = 0;
   for (auto& sg : segs) {
-    grids.push_back(mv_class_grid<T, ADJ>(std::get<0>(sg), std::get<2>(sg) - std::get<1>(sg)));
+    grids.push_back(mv_class_grid<T>(std::get<0>(sg), std::get<2>(sg) - std::get<1>(sg)));
     total += grids.back();
   }
   if (int rc = check_dot_ctas(a, total)) return rc;
@@ -917,15 +779,15 @@ static int launch_mv_t(const vbg_matrix* m, const ApplyArgs& a, const T* vals, c
     const int w0 = std::get<1>(segs[i]), w1 = std::get<2>(segs[i]);
     int rc = 0;
     switch (std::get<0>(segs[i])) {
-      case 1: rc = launch_mv_class<T, 1, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      case 2: rc = launch_mv_class<T, 2, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      case 3: rc = launch_mv_class<T, 3, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      case 4: rc = launch_mv_class<T, 4, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      case 5: rc = launch_mv_class<T, 5, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      case 6: rc = launch_mv_class<T, 6, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      case 7: rc = launch_mv_class<T, 7, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      case 8: rc = launch_mv_class<T, 8, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      default: rc = launch_mv_class<T, 0, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 1: rc = launch_mv_class<T, 1>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 2: rc = launch_mv_class<T, 2>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 3: rc = launch_mv_class<T, 3>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 4: rc = launch_mv_class<T, 4>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 5: rc = launch_mv_class<T, 5>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 6: rc = launch_mv_class<T, 6>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 7: rc = launch_mv_class<T, 7>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 8: rc = launch_mv_class<T, 8>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      default: rc = launch_mv_class<T, 0>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
     }
     if (rc) return rc;
     base += grids[i];
@@ -1272,7 +1134,8 @@ static int launch_fwd_mv(const vbg_matrix* m, const ApplyArgs& a, const T* v, cu
     if (pipe_use<T>(m, false, a, s, allow_alloc)) return launch_pipe_t<T>(m, a, s);
     if (!any) return kNotApplicable;
   }
-  return launch_mv_t<T, false>(m, a, v, s);
+  if constexpr (std::is_same<T, float>::value) return launch_mv_t<float>(m, a, v, s);
+  return launch_mma(m, false, a, s);
 }
 
 // The autotuner: the first forward multivector apply with a given leading
@@ -1306,7 +1169,9 @@ static int autotune_fwd(const vbg_matrix* m, const ApplyArgs& a0, const T* v, cu
   *choice = -1;
   auto* mm = const_cast<vbg_matrix*>(m);
   const auto cap_key = std::make_pair(a.ld, (int)sizeof(T));
-  for (int cand : {VBG_KERNEL_CHAIN, VBG_KERNEL_TILE, VBG_KERNEL_PIPE}) {
+  for (int cand : {VBG_KERNEL_CHAIN, VBG_KERNEL_TILE, VBG_KERNEL_PIPE, VBG_KERNEL_ROWS}) {
+    // alone on this apply, or FP32: rows run only what no other kernel takes
+    if (cand == VBG_KERNEL_ROWS && (std::is_same<T, float>::value || *choice < 0)) break;
     // the tiled kernel once per tile height cap (its own plan each) and per
     // tile order (fixed stride, work queue)
     for (int trial = 0; trial < 6; ++trial) {
@@ -1499,16 +1364,19 @@ static int launch_apply(const vbg_matrix* m, bool adj, bool f32, const ApplyArgs
     int rc = ensure_vals32(m, s);
     if (rc) return rc;
     const float* v = m->vals32.as<float>();
-    if (adj) return mv ? launch_mv_t<float, true>(m, a, v, s) : launch_vec_t<float, true>(m, a, v, s);
+    if (adj) {
+      VBG_CHECK(!mv, VBG_E_STATE, "FP32 multivectors have no adjoint apply");
+      return launch_vec_t<float, true>(m, a, v, s);
+    }
     return mv ? fwd(float{}, v) : launch_vec_t<float, false>(m, a, v, s);
   }
   if (m->dtype == VBG_C128) {
     const cplx* v = m->vals.as<cplx>();
-    if (adj) return mv ? launch_mv_t<cplx, true>(m, a, v, s) : launch_vec_t<cplx, true>(m, a, v, s);
+    if (adj) return mv ? launch_mma(m, true, a, s) : launch_vec_t<cplx, true>(m, a, v, s);
     return mv ? fwd(cplx{}, v) : launch_vec_t<cplx, false>(m, a, v, s);
   }
   const double* v = m->vals.as<double>();
-  if (adj) return mv ? launch_mv_t<double, true>(m, a, v, s) : launch_vec_t<double, true>(m, a, v, s);
+  if (adj) return mv ? launch_mma(m, true, a, s) : launch_vec_t<double, true>(m, a, v, s);
   return mv ? fwd(double{}, v) : launch_vec_t<double, false>(m, a, v, s);
 }
 

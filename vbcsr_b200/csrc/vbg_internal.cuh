@@ -76,6 +76,14 @@ __device__ __forceinline__ cplx cmad(double cr, double ci, cplx x, cplx b) {
   return {fma(cr, x.re, fma(-ci, x.im, b.re)), fma(cr, x.im, fma(ci, x.re, b.im))};
 }
 
+// D = A B + C for one 8 x 8 x 4 FP64 tile (mma.sync m8n8k4, row.col): lane l
+// holds A(l / 4, l % 4), B(l % 4, l / 4) and C(l / 4, 2 (l % 4) + {0, 1}).
+__device__ __forceinline__ void dmma_884(double& c0, double& c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+
 inline size_t elem_size(int dtype) { return dtype == VBG_C128 ? 16 : 8; }
 
 // ------------------------------------------------------------- device buffer

@@ -253,14 +253,6 @@ __device__ __forceinline__ double sq_mag(double v) { return __dmul_rn(v, v); }
 __device__ __forceinline__ double sq_mag(float v) { return __dmul_rn((double)v, (double)v); }
 __device__ __forceinline__ double sq_mag(cplx v) { return fma(v.re, v.re, __dmul_rn(v.im, v.im)); }
 
-// D = A B + C for one 8 x 8 x 4 FP64 tile (mma.sync m8n8k4, row.col): lane l
-// holds A(l / 4, l % 4), B(l % 4, l / 4) and C(l / 4, 2 (l % 4) + {0, 1}).
-__device__ __forceinline__ void dmma_884(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
-}
-
 // Accumulator of one C block C_ij (r x c, row-major) held by a warp.  Blocks
 // of at most 8 x 8 (R != 0) live in registers in the layout of the m8n8k4 C
 // fragment: lane l holds (l / 4, 2 (l % 4) + {0, 1}).  Real blocks multiply on
