@@ -129,34 +129,118 @@ __device__ __forceinline__ void vec_row(const ApplyArgs& a, const T* __restrict_
   vec_row_finish<T, R>(a, row, lane, acc, wred, d0, d1);
 }
 
-// Rows wider than 8: lane handles output rows o0 + lane over all entries.
+// Rows wider than 8 (outputs of one block row, or of one block column for
+// the adjoint), a warp per row: lane l = 8 rs + qs.  Forward, lane (rs, qs)
+// takes rows 4 v + rs and columns qs (mod 8) of every block, so the eight qs
+// lanes read a row's values side by side; the adjoint, where the outputs run
+// along a block's rows, takes outputs 8 v + qs and reads rows rs (mod 4).
+// Each X element is loaded once per lane for up to 32 outputs, and the eight
+// value loads of a round are independent.  What bounds it is the stream of
+// values; one lane per output row, as this was before, read a value per lane
+// at a stride of a whole block row (4000 rows of 9-20 complex, 168 MB:
+// forward 86 us, adjoint 166 us; the two together 250 us, now 126).
+// Entries sub, sub + split, ... of the row; returns this lane's output
+// o0 + lane's partial sum (forward: outputs permuted, see wide_out).
+template <bool ADJ>
+__device__ __forceinline__ int wide_out(int lane) {
+  return ADJ ? lane : 4 * (lane & 7) + (lane >> 3);
+}
+
+template <typename T, bool ADJ>
+__device__ __forceinline__ T vec_wide_sum(const ApplyArgs& a, const T* __restrict__ vals, int e0, int e1, int r,
+                                          int o0, int lane, int sub, int split) {
+  const T* __restrict__ x = static_cast<const T*>(a.X);
+  const int qs = lane & 7, rs = lane >> 3;
+  constexpr int V = ADJ ? 4 : 8;
+  T acc[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) acc[v] = zero_s<T>();
+  for (int base = e0 + sub; base < e1; base += 32 * split) {
+    const int cnt = min(32, (e1 - base + split - 1) / split);
+    long long xo = 0, vo = 0;
+    int in = 0;
+    if (lane < cnt) {
+      const int e = base + lane * split;
+      if (!ADJ && a.slot_meta) {
+        const int2 mt = __ldg(a.slot_meta + e);
+        xo = mt.x;
+        in = mt.y & 0xff;
+        vo = __ldg(a.blk_off + e);
+      } else {
+        const int src = __ldg(a.ent_src + e);
+        xo = a.scal_off[src];
+        in = a.bsz[src];
+        vo = a.blk_off[ADJ ? __ldg(a.ent_slot + e) : e];
+      }
+    }
+    for (int j = 0; j < cnt; ++j) {
+      const T* __restrict__ xp = x + __shfl_sync(0xffffffffu, xo, j);
+      const T* __restrict__ vp = vals + __shfl_sync(0xffffffffu, vo, j);
+      const int inner = __shfl_sync(0xffffffffu, in, j);
+      if constexpr (!ADJ) {
+        for (int q0 = 0; q0 < inner; q0 += 8) {
+          const int q = q0 + qs;
+          const bool kv = q < inner;
+          const T xv = kv ? xp[q] : zero_s<T>();
+          T av[V];
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            const int o = o0 + 4 * v + rs;
+            av[v] = kv && o < r ? vp[(int64_t)o * inner + q] : zero_s<T>();
+          }
+#pragma unroll
+          for (int v = 0; v < V; ++v) acc[v] = fma_s(av[v], xv, acc[v]);
+        }
+      } else {
+        for (int q0 = 0; q0 < inner; q0 += 8) {
+          T av[2][V], xv[2];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int q = q0 + 4 * h + rs;
+            const bool kv = q < inner;
+            xv[h] = kv ? xp[q] : zero_s<T>();
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+              const int o = o0 + 8 * v + qs;
+              av[h][v] = kv && o < r ? vp[(int64_t)q * r + o] : zero_s<T>();
+            }
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int v = 0; v < V; ++v) acc[v] = fma_s(conj_s(av[h][v]), xv[h], acc[v]);
+        }
+      }
+    }
+  }
+  // the lanes of an output meet by butterflies; each lane keeps its own output
+  T mine = zero_s<T>();
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    if (o0 + v * (32 / V) >= r) break;
+#pragma unroll
+    for (int off = ADJ ? 8 : 1; off < (ADJ ? 32 : 8); off <<= 1) acc[v] = add_s(acc[v], shfl_xor_s(acc[v], off));
+    if ((ADJ ? rs : qs) == v) mine = acc[v];
+  }
+  return mine;
+}
+
+template <typename T>
+__device__ __forceinline__ void vec_wide_finish(const ApplyArgs& a, T sum, int64_t gi, double& d0, double& d1) {
+  const T y = epi_value(a, sum, gi);
+  static_cast<T*>(a.Y)[gi] = y;
+  epi_finish(a, y, gi, d0, d1);
+}
+
 template <typename T, bool ADJ>
 __device__ void vec_row_wide(const ApplyArgs& a, const T* __restrict__ vals, int row, int lane, double& d0,
                              double& d1) {
   const int r = a.bsz[row];
   const int e0 = a.ptr[row], e1 = a.ptr[row + 1];
-  const T* __restrict__ x = static_cast<const T*>(a.X);
   for (int o0 = 0; o0 < r; o0 += 32) {
-    const int o = o0 + lane;
-    if (o < r) {
-      T acc = zero_s<T>();
-      for (int e = e0; e < e1; ++e) {
-        const int src = a.ent_src[e];
-        const int s = ADJ ? a.ent_slot[e] : e;
-        const int inner = a.bsz[src];
-        const T* xp = x + a.scal_off[src];
-        const T* ap = vals + a.blk_off[s] + (ADJ ? o : (int64_t)o * inner);
-        for (int q = 0; q < inner; ++q) {
-          T av = ap[ADJ ? (int64_t)q * r : q];
-          if (ADJ) av = conj_s(av);
-          acc = fma_s(av, xp[q], acc);
-        }
-      }
-      const int64_t gi = a.scal_off[row] + o;
-      const T y = epi_value(a, acc, gi);
-      static_cast<T*>(a.Y)[gi] = y;
-      epi_finish(a, y, gi, d0, d1);
-    }
+    const T sum = vec_wide_sum<T, ADJ>(a, vals, e0, e1, r, o0, lane, 0, 1);
+    const int o = o0 + wide_out<ADJ>(lane);
+    if (o < r) vec_wide_finish(a, sum, a.scal_off[row] + o, d0, d1);
   }
 }
 
@@ -370,6 +454,41 @@ __global__ void __launch_bounds__(kThreads) apply_vec_kernel(ApplyArgs a, const 
   if (a.want_dots) grid_reduce2(d0, d1, a.partials, a.counter, a.dots_out, part_base, total);
 }
 
+// Vectors on matrices whose blocks are all over 8: a kernel of its own (its
+// registers are not set by the narrow rows' paths), `split` warps of the CTA
+// per block row when there are too few rows to fill the SMs.
+template <typename T, bool ADJ>
+__global__ void __launch_bounds__(kThreads, 2) apply_vec_wide_kernel(ApplyArgs a, const T* __restrict__ vals,
+                                                                     int max_bs, int split, int part_base,
+                                                                     int total) {
+  __shared__ T red[kThreads];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int per_cta = kWarps / split, sub = warp % split;
+  double d0 = 0.0, d1 = 0.0;
+  for (int wb = blockIdx.x * per_cta; wb < a.n_rows; wb += gridDim.x * per_cta) {  // CTA-uniform
+    const int row = wb + warp / split;
+    const bool on = row < a.n_rows;
+    const int r = on ? a.bsz[row] : 0;
+    const int e0 = on ? a.ptr[row] : 0, e1 = on ? a.ptr[row + 1] : 0;
+    // the CTA's rows may differ in size: every warp takes the barriers of
+    // the matrix's largest block
+    for (int o0 = 0; o0 < max_bs; o0 += 32) {
+      T sum = zero_s<T>();
+      if (o0 < r) sum = vec_wide_sum<T, ADJ>(a, vals, e0, e1, r, o0, lane, sub, split);
+      if (split > 1) {
+        red[threadIdx.x] = sum;
+        __syncthreads();
+        if (sub == 0)
+          for (int w = 1; w < split; ++w) sum = add_s(sum, red[threadIdx.x + 32 * w]);
+        __syncthreads();
+      }
+      const int o = o0 + wide_out<ADJ>(lane);
+      if (sub == 0 && o < r) vec_wide_finish(a, sum, a.scal_off[row] + o, d0, d1);
+    }
+  }
+  if (a.want_dots) grid_reduce2(d0, d1, a.partials, a.counter, a.dots_out, part_base, total);
+}
+
 // FP32 multivectors the staged applies do not take: one launch per block-size
 // class; rows [w0, w1) of the class-ordered row list all have block size R
 // (R == 0: any size > 8).  FP64 and complex values run on vbg_mma.cu instead.
@@ -453,6 +572,21 @@ static int vec_max_grid() {
   if (!cached[dev]) {
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, apply_vec_kernel<T, ADJ>, kThreads, 0) != cudaSuccess ||
+        per_sm < 1)
+      per_sm = 1;
+    cached[dev] = per_sm * sm_count();
+  }
+  return cached[dev];
+}
+
+template <typename T, bool ADJ>
+static int vec_wide_max_grid() {
+  static int cached[kMaxDevices] = {};
+  const int dev = current_device();
+  if (!cached[dev]) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, apply_vec_wide_kernel<T, ADJ>, kThreads, 0) !=
+            cudaSuccess ||
         per_sm < 1)
       per_sm = 1;
     cached[dev] = per_sm * sm_count();
@@ -699,6 +833,16 @@ static int launch_vec_srow(const vbg_matrix* m, const ApplyArgs& a0, const T* va
 template <typename T, bool ADJ>
 static int launch_vec_t(const vbg_matrix* m, const ApplyArgs& a0, const T* vals, cudaStream_t s) {
   if (a0.srow) return launch_vec_srow<T, ADJ>(m, a0, vals, s);
+  if (m->min_bs > 8) {
+    // warps per row as the multivector rows take them (row_split)
+    const int split = row_split(m, m->n);
+    const int per_cta = kWarps / split;
+    const int wgrid = std::max(1, std::min((m->n + per_cta - 1) / per_cta, vec_wide_max_grid<T, ADJ>()));
+    if (int rc = check_dot_ctas(a0, wgrid)) return rc;
+    apply_vec_wide_kernel<T, ADJ><<<wgrid, kThreads, 0, s>>>(a0, vals, m->max_bs, split, 0, wgrid);
+    VBG_CUDA(cudaGetLastError());
+    return 0;
+  }
   const bool meta_only = !ADJ && a0.slot_meta && m->max_bs <= 8;
   const int wpc = meta_only ? kMetaWarps : kWarps;
   int grid = (a0.n_rows + wpc - 1) / wpc;

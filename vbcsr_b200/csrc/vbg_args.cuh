@@ -144,6 +144,18 @@ inline int check_dot_ctas(const ApplyArgs& a, int total) {
                   std::to_string(cap));
 }
 
+constexpr int kSplitWantWarps = 24;
+// Warps that share a task: the fewest of 1, 2, 4, 8 that give every SM
+// kSplitWantWarps warps (a warp alone walks its row's entries two at a time, so
+// a matrix of few rows otherwise waits on one row's loads), while each still
+// gets two entries of an average row.
+inline int row_split(const vbg_matrix* m, int64_t ntasks) {
+  const int64_t want = (int64_t)sm_count() * kSplitWantWarps;
+  int s = 1;
+  while (s < 8 && ntasks * s < want && m->nnzb >= 4 * (int64_t)s * m->n) s *= 2;
+  return s;
+}
+
 // The row-wise multivector apply on the FP64 tensor cores (vbg_mma.cu), FP64
 // and complex values.
 int launch_mma(const vbg_matrix* m, bool adj, const ApplyArgs& a, cudaStream_t s);

@@ -21,7 +21,7 @@
 // So every class of block sizes shares one launch (separate launches ran one
 // after the other), all 32 lanes work whatever the leading dimension, and a
 // block row's entries are split over up to eight warps of the CTA when there
-// are too few tasks to fill the SMs (mma_split).  Against the scalar
+// are too few tasks to fill the SMs (row_split).  Against the scalar
 // row-per-warp kernels, one launch per size class, that it replaces
 // (5000 block rows of 4-8, 24 columns: forward 270 us and adjoint 373 us of
 // five launches each; 4096 rows of 9-16, 16 columns: 175 us, now 54).  The
@@ -36,8 +36,6 @@
 namespace vbg {
 
 constexpr int kMmaWarps = 8;
-// Warps per SM that mma_split aims at.
-constexpr int kMmaWantWarps = 24;
 
 // The A operand of a lane: a real value, or a complex one.
 template <typename T> struct MmaA { double re; };
@@ -277,17 +275,6 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2)
   if (a.want_dots && !a.row_dots) grid_reduce2(d0, d1, a.partials, a.counter, a.dots_out, part_base, total);
 }
 
-// Warps that share a task: the fewest of 1, 2, 4, 8 that give every SM
-// kMmaWantWarps warps (a warp alone walks its row's entries two at a time, so
-// a matrix of few rows otherwise waits on one row's loads), while each still
-// gets two entries of an average row.
-static int mma_split(const vbg_matrix* m, int64_t ntasks) {
-  const int64_t want = (int64_t)sm_count() * kMmaWantWarps;
-  int s = 1;
-  while (s < kMmaWarps && ntasks * s < want && m->nnzb >= 4 * (int64_t)s * m->n) s *= 2;
-  return s;
-}
-
 template <typename T, int MT, int NP, bool ADJ>
 static int launch_mma_k(const vbg_matrix* m, const ApplyArgs& a, const T* vals, cudaStream_t s) {
   constexpr int W = std::is_same<T, cplx>::value ? 2 : 1;
@@ -296,7 +283,7 @@ static int launch_mma_k(const vbg_matrix* m, const ApplyArgs& a, const T* vals, 
   const int rgroups = (m->max_bs + 8 * MT - 1) / (8 * MT);
   const int cgroups = (int)(((int64_t)a.ld * W + 16 * NP - 1) / (16 * NP));
   const int64_t ntasks = (int64_t)a.n_rows * (a.row_dots ? 1 : (int64_t)rgroups * cgroups);
-  const int split = mma_split(m, ntasks);
+  const int split = row_split(m, ntasks);
   const int dev = current_device();
   int& occ = per_sm[dev][split > 1];
   if (!occ) {
