@@ -28,6 +28,7 @@ CUDA_SOURCES = [
     "vbg_vec.cu",
     "vbg_algebra.cu",
     "vbg_spgemm.cu",
+    "vbg_numeric.cu",
     "vbg_sddmm.cu",
     "vbg_struct.cu",
 ]

@@ -31,6 +31,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include "vbg_internal.cuh"
+#include "vbg_numeric.cuh"
 
 namespace vbg {
 
@@ -39,35 +40,12 @@ int block_norms_dev(const vbg_matrix* m, double* out, cudaStream_t s);
 constexpr int kEmpty = -1;
 constexpr int kSmemBudget = 96 * 1024;  // shared memory per CTA for the tables
 constexpr int kMaxWarps = 8;
+constexpr int64_t kSymTempMax = (int64_t)1 << 28;  // symbolic phase in one pass: columns of room (1 GB)
 constexpr int kNumItem = 8;    // C blocks per numeric work item
 constexpr int kPairBatch = 4;  // block pairs whose operands are loaded together
 constexpr int kNumWarpsCta = 8;  // warps of a numeric CTA
 constexpr long long kOffMask = (1ll << 56) - 1;  // pair list: offset bits below the inner size
 constexpr int kWinCap = 1024;    // numeric: entries of a warp's window table of A's row
-constexpr int kRowStageCap = 8192;  // numeric row kernel: A row values staged in shared memory (64 KB)
-
-// Pair gates.  kGateSum is the plain product (symbolic: keep j iff
-// sum_k |A_ik||B_kj| > threshold; numeric: skip a pair below threshold /
-// max(1, n_A)).  The others are the fused triple products' per-row gates
-// (ops/spmm/rarh.hpp, rhar.hpp, square_polynomial.hpp): a pair
-// (i,k)(k,j) reaches C's row only when |L_ik||R_kj| >= eps, and every column
-// a pair reaches is kept by the symbolic phase:
-//   kGateStage1  eps = thr / (2 max(1, n_L) |R row k| max|A|)   (T = L B)
-//   kGateStage2  eps = thr / (2 n_L), |L_ik| the stage-one bound  (C = T A)
-//   kGatePoly    eps = thr / max(1, n_L), 0 for an all-zero A      (A A)
-// with n_L the left operand's blocks in row i; every eps is 0 for thr <= 0.
-constexpr int kGateSum = 0;
-constexpr int kGateStage1 = 1;
-constexpr int kGateStage2 = 2;
-constexpr int kGatePoly = 3;
-
-__host__ __device__ inline double gate_eps(int mode, double thr, double amax, int nl, int nb) {
-  if (mode == kGateStage1)
-    return (thr > 0.0 && amax > 0.0 && nb > 0) ? thr / (2.0 * (double)(nl > 1 ? nl : 1) * (double)nb * amax) : 0.0;
-  if (mode == kGateStage2) return (thr > 0.0 && nl > 0) ? thr / (2.0 * (double)nl) : 0.0;
-  if (mode == kGatePoly) return (thr > 0.0 && amax > 0.0) ? thr / (double)(nl > 1 ? nl : 1) : 0.0;
-  return thr / (double)(nl > 1 ? nl : 1);
-}
 
 struct SymArgs {
   const int* a_rp;
@@ -82,10 +60,11 @@ struct SymArgs {
   const int* rows;    // rows of this bin
   int nrows;
   int T;              // table entries (power of two)
-  int pass;           // 0: count, 1: write sorted columns
-  int* cnt;           // [n] kept columns per row (pass 0)
-  const int* c_rp;    // pass 1
-  int* c_ci;          // pass 1
+  int count, write;   // store the kept columns' number, write them sorted
+  int* cnt;           // [n] kept columns per row (count)
+  const int* c_rp;    // where row i's columns go in c_ci (write), if tmp_off is nullptr
+  int* c_ci;
+  const int64_t* tmp_off;  // or where the row list's w-th row's columns go
   char* gtab;         // global tables (nullptr = shared memory)
   int* err;           // set on a table overflow (never expected)
   int mode;           // kGate*
@@ -112,8 +91,8 @@ __device__ __forceinline__ void bitonic_sort_warp(int* list, int L, int lane) {
   }
 }
 
-// Table layout per warp: keys int[T] | vals double[T] | list int[T/2]
-__host__ __device__ inline size_t sym_table_bytes(int T) { return (size_t)T * 12 + (size_t)(T / 2) * 4 + 16; }
+// Table layout per warp: vals double[T] | keys int[T] | list int[T]
+__host__ __device__ inline size_t sym_table_bytes(int T) { return (size_t)T * 16 + 16; }
 
 __global__ void spgemm_symbolic_kernel(SymArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -156,18 +135,33 @@ __global__ void spgemm_symbolic_kernel(SymArgs a) {
       }
       __syncwarp();
     }
-    for (int as = a.a_rp[row]; as < a.a_rp[row + 1]; ++as) {
-      const int kk = a.a_ci[as];
-      const double na = a.nA[as];
-      const int b0 = a.b_rp[kk], b1 = a.b_rp[kk + 1];
-      const double eps = a.mode != kGateSum ? gate_eps(a.mode, a.thr, amax, nl, b1 - b0) : 0.0;
-      const int width = a.serial_lanes ? 1 : 32;
-      for (int bc = b0; bc < b1; bc += width) {
-        const int b = bc + lane;
-        const double v = (lane < width && b < b1) ? __dmul_rn(na, a.nB[b]) : 0.0;
-        // gated modes: a pair below its gate does not reach the row
-        if (lane < width && b < b1 && !(a.upper && a.b_ci[b] < row) && (a.mode == kGateSum || !(v < eps))) {
-          const int j = a.b_ci[b];
+    // 32 of A's slots at a time: the lanes fetch a slot's norm and B row
+    // each, and the next slot's columns and norms are loaded while this one's
+    // are entered (a slot at a time, each waited for three dependent loads)
+    for (int base = a.a_rp[row]; base < a.a_rp[row + 1]; base += 32) {
+      const int cnt = min(32, a.a_rp[row + 1] - base);
+      int lb0 = 0, lb1 = 0;
+      double lna = 0.0;
+      if (lane < cnt) {
+        const int kk = a.a_ci[base + lane];
+        lna = a.nA[base + lane];
+        lb0 = a.b_rp[kk];
+        lb1 = a.b_rp[kk + 1];
+      }
+      int b0 = __shfl_sync(0xffffffffu, lb0, 0), b1 = __shfl_sync(0xffffffffu, lb1, 0);
+      int col = b0 + lane < b1 ? a.b_ci[b0 + lane] : 0;
+      double nb = b0 + lane < b1 ? a.nB[b0 + lane] : 0.0;
+      for (int t = 0; t < cnt; ++t) {
+        const int n0 = __shfl_sync(0xffffffffu, lb0, (t + 1) & 31), n1 = __shfl_sync(0xffffffffu, lb1, (t + 1) & 31);
+        const bool more = t + 1 < cnt && n0 + lane < n1;
+        const int ncol = more ? a.b_ci[n0 + lane] : 0;
+        const double nnb = more ? a.nB[n0 + lane] : 0.0;
+        const double na = __shfl_sync(0xffffffffu, lna, t);
+        const double eps = a.mode != kGateSum ? gate_eps(a.mode, a.thr, amax, nl, b1 - b0) : 0.0;
+        auto enter = [&](int j, double norm) {
+          const double v = __dmul_rn(na, norm);
+          // gated modes: a pair below its gate does not reach the row
+          if ((a.upper && j < row) || (a.mode != kGateSum && v < eps)) return;
           int h = j & mask;
           int probes = 0;
           while (true) {
@@ -189,10 +183,27 @@ __global__ void spgemm_symbolic_kernel(SymArgs a) {
               break;
             }
           }
+        };
+        for (int b = b0; b < b1; b += 32) {
+          if (b > b0) {
+            col = b + lane < b1 ? a.b_ci[b + lane] : 0;
+            nb = b + lane < b1 ? a.nB[b + lane] : 0.0;
+          }
+          if (!a.serial_lanes) {
+            if (b + lane < b1) enter(col, nb);
+          } else {
+            for (int l = 0; l < 32 && b + l < b1; ++l) {
+              if (lane == l) enter(col, nb);
+              __syncwarp();
+            }
+          }
         }
-        if (a.serial_lanes) __syncwarp();
+        __syncwarp();
+        b0 = n0;
+        b1 = n1;
+        col = ncol;
+        nb = nnb;
       }
-      __syncwarp();
     }
     // kept columns: sum > threshold (common.hpp:664); gated: every column reached
     int base_pos = 0;
@@ -200,21 +211,34 @@ __global__ void spgemm_symbolic_kernel(SymArgs a) {
       const int h = h0 + lane;
       const bool kept = keys[h] != kEmpty && (a.mode != kGateSum || vals[h] > a.thr);
       const unsigned bal = __ballot_sync(0xffffffffu, kept);
-      if (a.pass == 1 && kept) list[base_pos + __popc(bal & ((1u << lane) - 1u))] = keys[h];
+      if (a.write && kept) list[base_pos + __popc(bal & ((1u << lane) - 1u))] = keys[h];
       base_pos += __popc(bal);
     }
-    if (a.pass == 0) {
-      if (lane == 0) a.cnt[row] = base_pos;
-    } else if (base_pos > 0) {
+    if (a.count && lane == 0) a.cnt[row] = base_pos;
+    if (a.write && base_pos > 0) {
       int L = 1;
       while (L < base_pos) L <<= 1;
       for (int i = base_pos + lane; i < L; i += 32) list[i] = 0x7fffffff;
       __syncwarp();
       bitonic_sort_warp(list, L, lane);
-      int* out = a.c_ci + a.c_rp[row];
+      int* out = a.c_ci + (a.tmp_off ? a.tmp_off[w] : (int64_t)a.c_rp[row]);
       for (int i = lane; i < base_pos; i += 32) out[i] = list[i];
     }
     __syncwarp();
+  }
+}
+
+// Rows of sorted columns from their room in the temporary list (tmp_off, in
+// the order of `rows`) to C's pattern, a warp per row.
+__global__ void gather_columns_kernel(int nrows, const int* __restrict__ rows, const int64_t* __restrict__ tmp_off,
+                                      const int* __restrict__ tmp, const int* __restrict__ c_rp,
+                                      int* __restrict__ c_ci) {
+  const int lane = threadIdx.x & 31;
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < nrows; w += warps) {
+    const int row = rows[w], c0 = c_rp[row], n = c_rp[row + 1] - c0;
+    const int* in = tmp + tmp_off[w];
+    for (int i = lane; i < n; i += 32) c_ci[c0 + i] = in[i];
   }
 }
 
@@ -244,9 +268,6 @@ struct NumArgs {
   const int* b_rp;      // B's row pointers (kGateStage1 divides by B's row lengths)
   double* bound_out;    // per C slot: the sum of the norms of its kept pairs (nullptr: not wanted)
   int drop;             // keep flags from the finished blocks' norms (else every block is kept)
-  const int* perm;      // row kernel: C's rows in class order
-  const int* c_rp;      // row kernel: C's row pointers
-  int row_cap;          // row kernel: A row values staged in shared memory up to this many
 };
 
 __device__ __forceinline__ double sq_mag(double v) { return __dmul_rn(v, v); }
@@ -577,74 +598,6 @@ __global__ void __launch_bounds__(kNumWarpsCta * 32, 3) spgemm_numeric_kernel(Nu
   if (lane == 0 && prods) atomicAdd(a.products, prods);
 }
 
-// Numeric phase, a CTA per C row (FP64 tensor-core path, A and B without
-// repeated block columns): the row's A values (contiguous in A) are copied
-// into shared memory once and its window table is built once, then the
-// CTA's warps take the row's C blocks in turn and read A's fragments from
-// shared memory -- only B's blocks come from L2.  Rows of A longer than
-// row_cap values read A from global memory as the item kernel does.
-template <typename T, int R, bool GATED>
-__global__ void __launch_bounds__(kNumWarpsCta * 32, 3) spgemm_numeric_row_kernel(NumArgs a, const T* __restrict__ A,
-                                                                 const T* __restrict__ B, T* __restrict__ C) {
-  extern __shared__ __align__(16) unsigned char srow_raw[];
-  T* srow = reinterpret_cast<T*>(srow_raw);
-  __shared__ longlong2 plists[kNumWarpsCta][32];
-  __shared__ int wtab[kWinCap];
-  __shared__ int s_lo, s_hi;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  longlong2* plist = plists[warp];
-  unsigned long long prods = 0;
-  const double amax = GATED ? *a.amax : 0.0;
-  for (int w = a.w0 + blockIdx.x; w < a.w1; w += gridDim.x) {
-    const int row = a.perm[w];
-    const int c0 = a.c_rp[row], c1 = a.c_rp[row + 1];
-    if (c0 == c1) continue;
-    const int a0 = a.a_rp[row], a1 = a.a_rp[row + 1];
-    const long long aoff0 = a.a_off[a0], alen = a.a_off[a1] - aoff0;
-    const bool staged = alen <= (long long)a.row_cap;
-    __syncthreads();  // the previous row's reads of srow and wtab are done
-    if (threadIdx.x == 0) {
-      s_lo = INT32_MAX;
-      s_hi = -1;
-    }
-    if (staged)
-      for (long long e = threadIdx.x; e < alen; e += blockDim.x) srow[e] = A[aoff0 + e];
-    __syncthreads();
-    int lo = INT32_MAX, hi = -1;
-    for (int as = a0 + threadIdx.x; as < a1; as += blockDim.x) {
-      const int k = a.a_ci[as];
-      lo = min(lo, k);
-      hi = max(hi, k);
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, off));
-      hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, off));
-    }
-    if (lane == 0 && hi >= 0) {
-      atomicMin(&s_lo, lo);
-      atomicMax(&s_hi, hi);
-    }
-    __syncthreads();
-    const int kmin = s_lo;
-    const int span = (a1 > a0 && s_hi - kmin < kWinCap) ? s_hi - kmin + 1 : 0;
-    for (int t = threadIdx.x; t < span; t += blockDim.x) wtab[t] = -1;
-    __syncthreads();
-    if (span)
-      for (int as = a0 + threadIdx.x; as < a1; as += blockDim.x) wtab[a.a_ci[as] - kmin] = as;
-    __syncthreads();
-    const double row_eps = gate_eps(GATED ? a.mode : kGateSum, a.thr, amax, a1 - a0, 0);
-    // A's values at their offsets in A: the staged copy (generic loads that
-    // meet shared memory) or A itself
-    const T* Ab = staged ? reinterpret_cast<const T*>(reinterpret_cast<uintptr_t>(srow) -
-                                                      static_cast<uintptr_t>(aoff0) * sizeof(T))
-                         : A;
-    for (int p = c0 + warp; p < c1; p += kNumWarpsCta)
-      numeric_block<T, R, GATED>(a, Ab, B, C, p, R, a0, a1, kmin, span, wtab, plist, lane, row_eps, amax, prods);
-  }
-  if (lane == 0 && prods) atomicAdd(a.products, prods);
-}
-
 // FP32 product results into the FP64 values of C.
 __global__ void widen_f32_kernel(const float* __restrict__ in, double* __restrict__ out, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -660,30 +613,6 @@ static int launch_numeric_r(const NumArgs& x, int64_t max_items, const T* A, con
   const int64_t want = (max_items + kNumWarpsCta - 1) / kNumWarpsCta;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sm_count() * 16));
   const bool gated = x.mode != kGateSum || x.bound_out || !x.drop;
-  // FP64 tensor-core products: a CTA per C row, A's row in shared memory
-  // (measured 4.5 % faster on the McWeeny products; FP32 products, on
-  // scalar FMAs, ran 6 % slower this way and keep the item kernel)
-  if constexpr (std::is_same<T, double>::value && R != 0) {
-    if (x.window && x.perm) {
-      const NumArgs& xr = x;
-      const int rgrid = std::max(1, std::min(x.w1 - x.w0, sm_count() * 16));
-      const size_t smem = (size_t)x.row_cap * sizeof(double);
-      static bool attr[2][kMaxDevices] = {};
-      const int dev = current_device();
-      if (!attr[gated][dev]) {
-        VBG_CUDA(cudaFuncSetAttribute(gated ? spgemm_numeric_row_kernel<T, R, true>
-                                            : spgemm_numeric_row_kernel<T, R, false>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr[gated][dev] = true;
-      }
-      if (gated) {
-        spgemm_numeric_row_kernel<T, R, true><<<rgrid, kNumWarpsCta * 32, smem, s>>>(xr, A, B, C);
-      } else {
-        spgemm_numeric_row_kernel<T, R, false><<<rgrid, kNumWarpsCta * 32, smem, s>>>(xr, A, B, C);
-      }
-      return 0;
-    }
-  }
   if constexpr (std::is_same<T, float>::value) {
     if (gated) return fail(VBG_E_ARG, "gated products run in FP64 only");
     spgemm_numeric_kernel<T, R, false><<<grid, kNumWarpsCta * 32, 0, s>>>(x, A, B, C);
@@ -722,25 +651,40 @@ struct Bin {
   std::vector<int> rows;
 };
 
-// Groups rows by table size.
+// Groups rows by table size.  The bins' launches run one after the other, so
+// a bin too small to fill the SMs joins the next larger one (a few rows at
+// the ends of a band otherwise cost a launch of their own, 25 us for one
+// CTA), unless its tables would grow more than fourfold.
+constexpr size_t kSmallBin = 2048;
 static std::vector<Bin> make_bins(const std::vector<int64_t>& need) {
   std::map<int, std::vector<int>> by;
   for (size_t i = 0; i < need.size(); ++i)
-    if (need[i] >= 0) by[next_pow2(need[i])].push_back((int)i);
+    if (need[i] >= 0) by[next_pow2(need[i] & 0xffffffff)].push_back((int)i);
   std::vector<Bin> out;
-  for (auto& kv : by) out.push_back({kv.first, std::move(kv.second)});
+  for (auto it = by.begin(); it != by.end(); ++it) {
+    auto nx = std::next(it);
+    if (nx != by.end() && it->second.size() < kSmallBin && nx->first <= 4 * it->first) {
+      nx->second.insert(nx->second.end(), it->second.begin(), it->second.end());
+      continue;
+    }
+    out.push_back({it->first, std::move(it->second)});
+  }
   return out;
 }
 
-// Warp per row i of A: the symbolic table size of C's row i, 2 b + 1 with b
-// the least of n, the sum of the lengths of the B rows k that A's row
-// touches (common.hpp:600-616 sizes its tables by these two) and the span
-// of the column range those B rows cover (their columns are sorted); -1 for
-// an empty row.  `upper`: only columns >= i are inserted, so the span starts
-// at i at the earliest (-1 when every column lies below the row).
+// Warp per row i of A: what C's row i needs of the symbolic phase.  b, the
+// least of n, the sum of the lengths of the B rows k that A's row touches
+// (common.hpp:600-616 sizes its tables by these two) and the span of the
+// column range those B rows cover (their columns are sorted), bounds its
+// columns; the table needs 2 b + 1 entries, or the span where that is less:
+// columns of one span never collide in a table as large.  need[i] = b << 32 |
+// entries; -1 for an empty row; *pairs the sum of those lengths.  `upper`: only columns >= i are inserted, so
+// the span starts at i at the earliest (-1 when every column lies below the
+// row).
 __global__ void sym_need_kernel(int n, const int* __restrict__ a_rp, const int* __restrict__ a_ci,
                                 const int* __restrict__ b_rp, const int* __restrict__ b_ci, int upper,
-                                int self_cols, int64_t* __restrict__ need) {
+                                int self_cols, int64_t* __restrict__ need,
+                                unsigned long long* __restrict__ pairs) {
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
@@ -772,10 +716,11 @@ __global__ void sym_need_kernel(int n, const int* __restrict__ a_rp, const int* 
       hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, off));
     }
     if (lane == 0) {
+      if (bound) atomicAdd(pairs, (unsigned long long)bound);
       if (upper) lo = max(lo, i);
       const long long span = (long long)hi - lo + 1;
       const long long b = min(min(bound, (long long)n), span);
-      need[i] = (bound == 0 || span <= 0) ? -1 : 2 * b + 1;
+      need[i] = (bound == 0 || span <= 0) ? -1 : (b << 32) | min(2 * b + 1, span);
     }
   }
 }
@@ -800,32 +745,27 @@ __global__ void item_fill_kernel(int n, const int* __restrict__ perm, const int*
   }
 }
 
+// Launches per bin over the rows listed in rows_dev, bin after bin.
 template <typename F>
-static int launch_binned(const std::vector<Bin>& bins, size_t (*table_bytes)(int), DevBuf& rows_dev, DevBuf& gtab,
-                         cudaStream_t s, F&& launch) {
-  size_t total_rows = 0;
-  for (auto& b : bins) total_rows += b.rows.size();
-  std::vector<int> all;
-  all.reserve(total_rows);
-  for (auto& b : bins) all.insert(all.end(), b.rows.begin(), b.rows.end());
-  int rc = rows_dev.ensure(std::max<size_t>(all.size(), 1) * sizeof(int));
-  if (rc) return rc;
-  if (!all.empty()) VBG_CUDA(cudaMemcpyAsync(rows_dev.p, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+static int launch_binned(const std::vector<Bin>& bins, size_t (*table_bytes)(int), const DevBuf& rows_dev, DevBuf& gtab,
+                         F&& launch) {
+  int rc;
   size_t off = 0;
   for (auto& b : bins) {
     const size_t tb = table_bytes(b.T);
     const int nrows = (int)b.rows.size();
     const int* rows = rows_dev.as<int>() + off;
+    const size_t first = off;
     off += b.rows.size();
     if (tb <= (size_t)kSmemBudget) {
       const int wpb = (int)std::max<size_t>(1, std::min<size_t>(kMaxWarps, kSmemBudget / tb));
       const int grid = std::max(1, std::min((nrows + wpb - 1) / wpb, sm_count() * 8));
-      if ((rc = launch(rows, nrows, b.T, grid, wpb, (size_t)wpb * tb, (char*)nullptr))) return rc;
+      if ((rc = launch(rows, first, nrows, b.T, grid, wpb, (size_t)wpb * tb, (char*)nullptr))) return rc;
     } else {
       const int wpb = 4;
       const int grid = std::max(1, std::min((nrows + wpb - 1) / wpb, sm_count() * 2));
       if ((rc = gtab.ensure((size_t)grid * wpb * tb))) return rc;
-      if ((rc = launch(rows, nrows, b.T, grid, wpb, (size_t)0, gtab.as<char>()))) return rc;
+      if ((rc = launch(rows, first, nrows, b.T, grid, wpb, (size_t)0, gtab.as<char>()))) return rc;
     }
   }
   return 0;
@@ -848,130 +788,19 @@ struct GateSpec {
   bool self_cols = false;               // kGatePoly: A's columns and the diagonal join every row
 };
 
-// The thresholded product C = A B; with `upper`, only its block columns at
-// or above each row (the symbolic phase skips the others, and the numeric
-// phase follows C's pattern).
-static int spgemm_run(const vbg_matrix* A, const vbg_matrix* B, double thr, int upper, vbg_matrix** Cout,
-                      int64_t* stats, cudaStream_t s, int precision = VBG_PREC_F64,
-                      const GateSpec& gate = GateSpec{}) {
-  VBG_CHECK(A && B && Cout, VBG_E_ARG, "null argument");
-  VBG_CHECK(A->dtype == B->dtype, VBG_E_ARG, "A and B must have the same dtype");
-  VBG_CHECK(precision == VBG_PREC_F64 || (precision == VBG_PREC_F32 && A->dtype == VBG_F64), VBG_E_ARG,
-            "precision must be VBG_PREC_F64, or VBG_PREC_F32 for real matrices");
-  VBG_CHECK(A->n == B->n && A->h_bsz == B->h_bsz, VBG_E_ARG, "spmm: A's columns and B's rows differ");
-  const int n = A->n;
+// The numeric phase of the products vbg_numeric.cu does not take: FP32
+// values, blocks over 8, repeated block columns, rows too long for its
+// shared memory.  B's column view is built.
+static int numeric_items(const vbg_matrix* A, const vbg_matrix* B, vbg_matrix* C, const double* normsA,
+                         const double* normsB, const NumericGate& gate, int precision, unsigned char* keep,
+                         unsigned long long* products, cudaStream_t s) {
+  const int n = C->n;
+  const int64_t cnnzb = C->nnzb;
+  const bool small = std::max(A->max_bs, B->max_bs) <= 8;
   int rc;
-  // block norms of both operands (cached per call)
-  DevBuf nA(s), nB(s), cnt(s), err(s), gtab(s), rows_dev(s);
-  const double* normsA = gate.left_norms;
-  const double* normsB = gate.right_norms;
-  if (!normsA) {
-    if ((rc = nA.ensure(std::max<int64_t>(A->nnzb, 1) * 8))) return rc;
-    if ((rc = block_norms_dev(A, nA.as<double>(), s))) return rc;
-    normsA = nA.as<double>();
-  }
-  if (!normsB) {
-    if ((rc = nB.ensure(std::max<int64_t>(B->nnzb, 1) * 8))) return rc;
-    if ((rc = block_norms_dev(B, nB.as<double>(), s))) return rc;
-    normsB = nB.as<double>();
-  }
-  VBG_CHECK(gate.mode == kGateSum || gate.amax, VBG_E_ARG, "gated product without the operand's largest norm");
-  VBG_CHECK(!(gate.bound_out && gate.drop), VBG_E_ARG, "pair-norm bounds of a dropped product");
-  if ((rc = cnt.ensure((n + 1) * sizeof(int)))) return rc;
-  if ((rc = err.ensure(16))) return rc;
-  VBG_CUDA(cudaMemsetAsync(err.p, 0, 16, s));
-  VBG_CUDA(cudaMemsetAsync(cnt.p, 0, (n + 1) * sizeof(int), s));
-  const int serial_b = B->dup_cols ? 1 : 0;
-
-  // symbolic table sizes, computed on the device (sym_need_kernel)
-  // page-locked staging of this thread's calls (each use completes before
-  // the call returns)
-  thread_local HostBuf h_rows;
-  std::vector<int64_t> need(n, -1);
-  if (n) {
-    DevBuf dneed(s);
-    if ((rc = dneed.ensure(n * sizeof(int64_t)))) return rc;
-    if ((rc = h_rows.ensure(n * sizeof(int64_t)))) return rc;
-    const int g = std::max(1, std::min((n + 7) / 8, sm_count() * 16));
-    sym_need_kernel<<<g, 256, 0, s>>>(n, A->row_ptr.as<int>(), A->col_ind.as<int>(), B->row_ptr.as<int>(),
-                                      B->col_ind.as<int>(), upper, gate.self_cols ? 1 : 0, dneed.as<int64_t>());
-    VBG_CUDA(cudaGetLastError());
-    VBG_CUDA(cudaMemcpyAsync(h_rows.p, dneed.p, n * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    VBG_CUDA(cudaStreamSynchronize(s));
-    std::memcpy(need.data(), h_rows.p, n * sizeof(int64_t));
-  }
-  auto sym_bins = make_bins(need);
-  SymArgs sa{};
-  sa.a_rp = A->row_ptr.as<int>();
-  sa.a_ci = A->col_ind.as<int>();
-  sa.nA = normsA;
-  sa.b_rp = B->row_ptr.as<int>();
-  sa.b_ci = B->col_ind.as<int>();
-  sa.nB = normsB;
-  sa.mode = gate.mode;
-  sa.amax = gate.amax;
-  sa.self_cols = gate.self_cols ? 1 : 0;
-  sa.thr = thr;
-  sa.serial_lanes = serial_b;
-  sa.upper = upper;
-  sa.cnt = cnt.as<int>();
-  sa.err = err.as<int>();
-  auto sym_launch = [&](int pass, const int* c_rp, int* c_ci) {
-    return launch_binned(sym_bins, sym_tb, rows_dev, gtab, s,
-                         [&](const int* rows, int nrows, int T, int grid, int wpb, size_t smem, char* gt) -> int {
-                           SymArgs x = sa;
-                           x.rows = rows;
-                           x.nrows = nrows;
-                           x.T = T;
-                           x.pass = pass;
-                           x.c_rp = c_rp;
-                           x.c_ci = c_ci;
-                           x.gtab = gt;
-                           if (smem > 48 * 1024)
-                             VBG_CUDA(cudaFuncSetAttribute(spgemm_symbolic_kernel,
-                                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-                           spgemm_symbolic_kernel<<<grid, wpb * 32, smem, s>>>(x);
-                           VBG_CUDA(cudaGetLastError());
-                           return 0;
-                         });
-  };
-  if ((rc = sym_launch(0, nullptr, nullptr))) return rc;
-  // C's row pointers: exclusive scan of the per-row counts on the device
-  DevBuf d_crp(s), d_cci(s), scan_tmp(s);
-  if ((rc = d_crp.ensure((n + 1) * sizeof(int)))) return rc;
-  size_t scan_bytes = 0;
-  VBG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, cnt.as<int>(), d_crp.as<int>(), n + 1, s));
-  if ((rc = scan_tmp.ensure(std::max<size_t>(scan_bytes, 16)))) return rc;
-  VBG_CUDA(cub::DeviceScan::ExclusiveSum(scan_tmp.p, scan_bytes, cnt.as<int>(), d_crp.as<int>(), n + 1, s));
-  int cnnzb_i = 0;
-  VBG_CUDA(cudaMemcpyAsync(&cnnzb_i, d_crp.as<int>() + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-  VBG_CUDA(cudaStreamSynchronize(s));
-  const int64_t cnnzb = cnnzb_i;
-  if ((rc = d_cci.ensure(std::max<int64_t>(cnnzb, 1) * sizeof(int)))) return rc;
-  if ((rc = sym_launch(1, d_crp.as<int>(), d_cci.as<int>()))) return rc;
-  int herr[4] = {0, 0, 0, 0};
-  VBG_CUDA(cudaMemcpyAsync(herr, err.p, 16, cudaMemcpyDeviceToHost, s));
-  VBG_CUDA(cudaStreamSynchronize(s));
-  VBG_CHECK(herr[0] == 0, VBG_E_DEVICE, "Hash table full in symbolic phase");
-
-  // result matrix on the symbolic pattern (rows sorted by the symbolic
-  // kernel); its structure metadata is built on the device
-  auto C = std::make_unique<vbg_matrix>();
-  C->dtype = A->dtype;
-  C->device = A->device;
-  if ((rc = adopt_device_structure(C.get(), A, d_crp, d_cci, cnnzb, s))) return rc;
-  C->dup_cols = false;  // the symbolic phase lists distinct columns
-  const size_t es = elem_size(C->dtype);
-  if ((rc = C->vals.ensure(std::max<int64_t>(C->nnz, 1) * es, s))) return rc;
-  DevBuf keep(s), prods(s);
-  if ((rc = keep.ensure(std::max<int64_t>(cnnzb, 1)))) return rc;
-  if ((rc = prods.ensure(16))) return rc;
-  VBG_CUDA(cudaMemsetAsync(prods.p, 0, 16, s));
-
   // numeric work items on the device, rows in class order (C has A's rows and
   // their grouping by block size); one launch per class of block sizes <= 8,
   // else one launch over all rows
-  const bool small = std::max(A->max_bs, B->max_bs) <= 8;
   const int64_t max_items = cnnzb / kNumItem + n;
   DevBuf items(s), istart(s), icnt(s);
   if ((rc = items.ensure(std::max<int64_t>(max_items, 1) * sizeof(int4)))) return rc;
@@ -999,7 +828,6 @@ static int spgemm_run(const vbg_matrix* A, const vbg_matrix* B, double thr, int 
   } else if (n) {
     launches.push_back({0, 0, n});
   }
-  if ((rc = build_csc_dev(B, s))) return rc;
   NumArgs na{};
   na.a_rp = A->row_ptr.as<int>();
   na.a_ci = A->col_ind.as<int>();
@@ -1013,22 +841,16 @@ static int spgemm_run(const vbg_matrix* A, const vbg_matrix* B, double thr, int 
   na.mode = gate.mode;
   na.amax = gate.amax;
   na.b_rp = B->row_ptr.as<int>();
-  na.drop = gate.drop ? 1 : 0;
-  if (gate.bound_out) {
-    if ((rc = gate.bound_out->ensure(std::max<int64_t>(cnnzb, 1) * sizeof(double)))) return rc;
-    na.bound_out = gate.bound_out->as<double>();
-  }
+  na.drop = gate.drop;
+  na.bound_out = gate.bound_out;
   na.bsz = A->bsz.as<int>();
   na.c_ci = C->col_ind.as<int>();
   na.c_off = C->blk_off.as<int64_t>();
-  na.thr = thr;
+  na.thr = gate.thr;
   na.dup = B->dup_cols ? 1 : 0;
   na.window = (A->dup_cols || B->dup_cols) ? 0 : 1;
-  na.perm = C->row_perm.as<int>();
-  na.c_rp = C->row_ptr.as<int>();
-  na.row_cap = kRowStageCap;
-  na.keep = keep.as<unsigned char>();
-  na.products = prods.as<unsigned long long>();
+  na.keep = keep;
+  na.products = products;
   {
     DevBuf c32(s);
     const bool f32 = precision == VBG_PREC_F32;
@@ -1063,6 +885,198 @@ static int spgemm_run(const vbg_matrix* A, const vbg_matrix* B, double thr, int 
       VBG_CUDA(cudaGetLastError());
     }
   }
+  return 0;
+}
+
+// The thresholded product C = A B; with `upper`, only its block columns at
+// or above each row (the symbolic phase skips the others, and the numeric
+// phase follows C's pattern).
+static int spgemm_run(const vbg_matrix* A, const vbg_matrix* B, double thr, int upper, vbg_matrix** Cout,
+                      int64_t* stats, cudaStream_t s, int precision = VBG_PREC_F64,
+                      const GateSpec& gate = GateSpec{}) {
+  VBG_CHECK(A && B && Cout, VBG_E_ARG, "null argument");
+  VBG_CHECK(A->dtype == B->dtype, VBG_E_ARG, "A and B must have the same dtype");
+  VBG_CHECK(precision == VBG_PREC_F64 || (precision == VBG_PREC_F32 && A->dtype == VBG_F64), VBG_E_ARG,
+            "precision must be VBG_PREC_F64, or VBG_PREC_F32 for real matrices");
+  VBG_CHECK(A->n == B->n && A->h_bsz == B->h_bsz, VBG_E_ARG, "spmm: A's columns and B's rows differ");
+  const int n = A->n;
+  int rc;
+  // block norms of both operands (cached per call)
+  DevBuf nA(s), nB(s), cnt(s), err(s), gtab(s), rows_dev(s);
+  const double* normsA = gate.left_norms;
+  const double* normsB = gate.right_norms;
+  if (!normsA) {
+    if ((rc = nA.ensure(std::max<int64_t>(A->nnzb, 1) * 8))) return rc;
+    if ((rc = block_norms_dev(A, nA.as<double>(), s))) return rc;
+    normsA = nA.as<double>();
+  }
+  if (!normsB && A == B && !gate.left_norms) normsB = normsA;  // a square
+  if (!normsB) {
+    if ((rc = nB.ensure(std::max<int64_t>(B->nnzb, 1) * 8))) return rc;
+    if ((rc = block_norms_dev(B, nB.as<double>(), s))) return rc;
+    normsB = nB.as<double>();
+  }
+  VBG_CHECK(gate.mode == kGateSum || gate.amax, VBG_E_ARG, "gated product without the operand's largest norm");
+  VBG_CHECK(!(gate.bound_out && gate.drop), VBG_E_ARG, "pair-norm bounds of a dropped product");
+  if ((rc = cnt.ensure((n + 1) * sizeof(int)))) return rc;
+  // {table overflow, -, largest merged A rows (entries, values), pairs (64 bits)}
+  if ((rc = err.ensure(24))) return rc;
+  VBG_CUDA(cudaMemsetAsync(err.p, 0, 24, s));
+  VBG_CUDA(cudaMemsetAsync(cnt.p, 0, (n + 1) * sizeof(int), s));
+  const int serial_b = B->dup_cols ? 1 : 0;
+
+  // symbolic table sizes, computed on the device (sym_need_kernel)
+  // page-locked staging of this thread's calls (each use completes before
+  // the call returns)
+  thread_local HostBuf h_rows;
+  std::vector<int64_t> need(n, -1);
+  if (n) {
+    DevBuf dneed(s);
+    if ((rc = dneed.ensure(n * sizeof(int64_t)))) return rc;
+    if ((rc = h_rows.ensure(n * sizeof(int64_t)))) return rc;
+    const int g = std::max(1, std::min((n + 7) / 8, sm_count() * 16));
+    sym_need_kernel<<<g, 256, 0, s>>>(n, A->row_ptr.as<int>(), A->col_ind.as<int>(), B->row_ptr.as<int>(),
+                                      B->col_ind.as<int>(), upper, gate.self_cols ? 1 : 0, dneed.as<int64_t>(),
+                                      reinterpret_cast<unsigned long long*>(err.as<int>() + 4));
+    VBG_CUDA(cudaGetLastError());
+    VBG_CUDA(cudaMemcpyAsync(h_rows.p, dneed.p, n * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    VBG_CUDA(cudaStreamSynchronize(s));
+    std::memcpy(need.data(), h_rows.p, n * sizeof(int64_t));
+  }
+  auto sym_bins = make_bins(need);
+  // the bins' rows, and where each may put its columns: room for as many as
+  // its bound (sym_need_kernel) allows, in one temporary list, so that one pass counts
+  // and writes them (a second pass over the pairs cost as much again: 190 of
+  // 325 us on 12000 rows of 29 blocks).  Products whose bounds add up to more
+  // than kSymTempMax columns count first and write in a second pass.
+  std::vector<int> sym_rows;
+  std::vector<int64_t> sym_off;
+  int64_t sym_room = 0;
+  for (auto& b : sym_bins)
+    for (int i : b.rows) {
+      sym_rows.push_back(i);
+      sym_off.push_back(sym_room);
+      sym_room += need[i] >> 32;
+    }
+  const bool one_pass = sym_room <= kSymTempMax;
+  DevBuf sym_tmp(s), sym_off_dev(s);
+  if ((rc = rows_dev.ensure(std::max<size_t>(sym_rows.size(), 1) * sizeof(int)))) return rc;
+  if (!sym_rows.empty())
+    VBG_CUDA(cudaMemcpyAsync(rows_dev.p, sym_rows.data(), sym_rows.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+  if (one_pass && !sym_rows.empty()) {
+    if ((rc = sym_tmp.ensure(std::max<int64_t>(sym_room, 1) * sizeof(int)))) return rc;
+    if ((rc = sym_off_dev.ensure(sym_off.size() * sizeof(int64_t)))) return rc;
+    VBG_CUDA(cudaMemcpyAsync(sym_off_dev.p, sym_off.data(), sym_off.size() * sizeof(int64_t), cudaMemcpyHostToDevice,
+                             s));
+  }
+  SymArgs sa{};
+  sa.a_rp = A->row_ptr.as<int>();
+  sa.a_ci = A->col_ind.as<int>();
+  sa.nA = normsA;
+  sa.b_rp = B->row_ptr.as<int>();
+  sa.b_ci = B->col_ind.as<int>();
+  sa.nB = normsB;
+  sa.mode = gate.mode;
+  sa.amax = gate.amax;
+  sa.self_cols = gate.self_cols ? 1 : 0;
+  sa.thr = thr;
+  sa.serial_lanes = serial_b;
+  sa.upper = upper;
+  sa.cnt = cnt.as<int>();
+  sa.err = err.as<int>();
+  auto sym_launch = [&](int count, int write, const int* c_rp, int* c_ci, const int64_t* tmp_off) {
+    return launch_binned(sym_bins, sym_tb, rows_dev, gtab,
+                         [&](const int* rows, size_t first, int nrows, int T, int grid, int wpb, size_t smem,
+                             char* gt) -> int {
+                           SymArgs x = sa;
+                           x.rows = rows;
+                           x.nrows = nrows;
+                           x.T = T;
+                           x.count = count;
+                           x.write = write;
+                           x.c_rp = c_rp;
+                           x.c_ci = c_ci;
+                           x.tmp_off = tmp_off ? tmp_off + first : nullptr;
+                           x.gtab = gt;
+                           if (smem > 48 * 1024)
+                             VBG_CUDA(cudaFuncSetAttribute(spgemm_symbolic_kernel,
+                                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                           spgemm_symbolic_kernel<<<grid, wpb * 32, smem, s>>>(x);
+                           VBG_CUDA(cudaGetLastError());
+                           return 0;
+                         });
+  };
+  if ((rc = sym_launch(1, one_pass ? 1 : 0, nullptr, sym_tmp.as<int>(), sym_off_dev.as<int64_t>()))) return rc;
+  // C's row pointers: exclusive scan of the per-row counts on the device
+  DevBuf d_crp(s), d_cci(s), scan_tmp(s);
+  if ((rc = d_crp.ensure((n + 1) * sizeof(int)))) return rc;
+  size_t scan_bytes = 0;
+  VBG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, cnt.as<int>(), d_crp.as<int>(), n + 1, s));
+  if ((rc = scan_tmp.ensure(std::max<size_t>(scan_bytes, 16)))) return rc;
+  VBG_CUDA(cub::DeviceScan::ExclusiveSum(scan_tmp.p, scan_bytes, cnt.as<int>(), d_crp.as<int>(), n + 1, s));
+  // the tensor-core numeric phase (vbg_numeric.cu) takes small blocks without
+  // repeated block columns; its merged A rows' sizes decide its launch
+  const bool small = std::max(A->max_bs, B->max_bs) <= 8;
+  const bool pairs = small && precision == VBG_PREC_F64 && !A->dup_cols && !B->dup_cols;
+  RowPairs ka(s);
+  struct {
+    int k, vals;
+    unsigned long long pairs;
+  } pair_max = {0, 0, 0};
+  if (pairs) {
+    if ((rc = merge_row_pairs(A, ka, err.as<int>() + 2, s))) return rc;
+    VBG_CUDA(cudaMemcpyAsync(&pair_max, err.as<int>() + 2, sizeof(pair_max), cudaMemcpyDeviceToHost, s));
+  }
+  int cnnzb_i = 0;
+  VBG_CUDA(cudaMemcpyAsync(&cnnzb_i, d_crp.as<int>() + n, sizeof(int), cudaMemcpyDeviceToHost, s));
+  VBG_CUDA(cudaStreamSynchronize(s));
+  const int64_t cnnzb = cnnzb_i;
+  if ((rc = d_cci.ensure(std::max<int64_t>(cnnzb, 1) * sizeof(int)))) return rc;
+  if (!one_pass) {
+    if ((rc = sym_launch(0, 1, d_crp.as<int>(), d_cci.as<int>(), nullptr))) return rc;
+  } else if (!sym_rows.empty()) {
+    const int nr = (int)sym_rows.size();
+    gather_columns_kernel<<<std::max(1, std::min((nr + 7) / 8, sm_count() * 16)), 256, 0, s>>>(
+        nr, rows_dev.as<int>(), sym_off_dev.as<int64_t>(), sym_tmp.as<int>(), d_crp.as<int>(), d_cci.as<int>());
+    VBG_CUDA(cudaGetLastError());
+  }
+  int herr[4] = {0, 0, 0, 0};
+  VBG_CUDA(cudaMemcpyAsync(herr, err.p, 16, cudaMemcpyDeviceToHost, s));
+  VBG_CUDA(cudaStreamSynchronize(s));
+  VBG_CHECK(herr[0] == 0, VBG_E_DEVICE, "Hash table full in symbolic phase");
+
+  // result matrix on the symbolic pattern (rows sorted by the symbolic
+  // kernel); its structure metadata is built on the device
+  auto C = std::make_unique<vbg_matrix>();
+  C->dtype = A->dtype;
+  C->device = A->device;
+  if ((rc = adopt_device_structure(C.get(), A, d_crp, d_cci, cnnzb, s))) return rc;
+  C->dup_cols = false;  // the symbolic phase lists distinct columns
+  const size_t es = elem_size(C->dtype);
+  if ((rc = C->vals.ensure(std::max<int64_t>(C->nnz, 1) * es, s))) return rc;
+  DevBuf keep(s), prods(s);
+  if ((rc = keep.ensure(std::max<int64_t>(cnnzb, 1)))) return rc;
+  if ((rc = prods.ensure(16))) return rc;
+  VBG_CUDA(cudaMemsetAsync(prods.p, 0, 16, s));
+
+  if ((rc = build_csc_dev(B, s))) return rc;
+  NumericGate ng;
+  ng.mode = gate.mode;
+  ng.amax = gate.amax;
+  ng.thr = thr;
+  ng.drop = gate.drop ? 1 : 0;
+  if (gate.bound_out) {
+    if ((rc = gate.bound_out->ensure(std::max<int64_t>(cnnzb, 1) * sizeof(double)))) return rc;
+    ng.bound_out = gate.bound_out->as<double>();
+  }
+  rc = kNumericNotFit;
+  if (pairs)
+    rc = numeric_pairs(A, B, C.get(), ka, pair_max.k, pair_max.vals,
+                       (double)pair_max.pairs * (upper ? 0.5 : 1.0), normsA, normsB, ng, keep.as<unsigned char>(),
+                       prods.as<unsigned long long>(), s);
+  if (rc == kNumericNotFit)
+    rc = numeric_items(A, B, C.get(), normsA, normsB, ng, precision, keep.as<unsigned char>(),
+                       prods.as<unsigned long long>(), s);
   if (rc) return rc;
   const int64_t sym_blocks = cnnzb;
   if (gate.drop && thr > 0.0 && (rc = compact_by_mask_dev(C.get(), keep.as<unsigned char>(), s))) return rc;

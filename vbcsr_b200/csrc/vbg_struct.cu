@@ -531,15 +531,51 @@ __global__ void compact_pattern_kernel(int n, const int* __restrict__ rp, const 
   for (int64_t i = tid; i <= n; i += stride) new_rp[i] = pos[rp[i]];
 }
 
+// Copies the kept blocks.  A warp takes 32 of them: the lanes fetch one
+// block's source slot, offsets and length each (three dependent loads, once
+// for 32 blocks instead of once per block), then the warp copies the blocks
+// four at a time with all their loads issued before the stores.  Bound by
+// HBM: 830k blocks of 4-8 (240 MB in, 240 MB out).
 template <typename T>
-__global__ void gather_blocks_kernel(int64_t nout, const int* __restrict__ old_of, const int64_t* __restrict__ old_off,
-                                     const T* __restrict__ src, const int64_t* __restrict__ new_off,
-                                     T* __restrict__ dst) {
+__global__ void __launch_bounds__(256) gather_blocks_kernel(int64_t nout, const int* __restrict__ old_of,
+                                                            const int64_t* __restrict__ old_off,
+                                                            const T* __restrict__ src,
+                                                            const int64_t* __restrict__ new_off,
+                                                            T* __restrict__ dst) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t k = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); k < nout; k += warps) {
-    const int64_t o = old_off[old_of[k]], d = new_off[k], len = new_off[k + 1] - d;
-    for (int64_t e = lane; e < len; e += 32) dst[d + e] = src[o + e];
+  for (int64_t k0 = 32 * (blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5)); k0 < nout;
+       k0 += 32 * warps) {
+    long long o = 0, d = 0, len = 0;
+    if (k0 + lane < nout) {
+      d = new_off[k0 + lane];
+      len = new_off[k0 + lane + 1] - d;
+      o = old_off[old_of[k0 + lane]];
+    }
+    const int cnt = (int)min((int64_t)32, nout - k0);
+    for (int j = 0; j < cnt; j += 4) {
+      const T* sp[4];
+      T* dp[4];
+      long long n[4];
+      T v[4][2];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        // past the last block: nothing (a lane without a block has length 0)
+        sp[u] = src + __shfl_sync(0xffffffffu, o, (j + u) & 31);
+        dp[u] = dst + __shfl_sync(0xffffffffu, d, (j + u) & 31);
+        n[u] = __shfl_sync(0xffffffffu, len, (j + u) & 31);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (lane + 32 * h < n[u]) v[u][h] = sp[u][lane + 32 * h];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (lane + 32 * h < n[u]) dp[u][lane + 32 * h] = v[u][h];
+        for (long long e = 64 + lane; e < n[u]; e += 32) dp[u][e] = sp[u][e];
+      }
+    }
   }
 }
 
@@ -573,7 +609,7 @@ int compact_by_mask_dev(vbg_matrix* m, const unsigned char* keep, cudaStream_t s
   const size_t es = elem_size(d->dtype);
   if ((rc = d->vals.ensure(std::max<int64_t>(d->nnz, 1) * es, s))) return rc;
   if (kept) {
-    const int g2 = (int)std::max<int64_t>(1, std::min<int64_t>((kept + 7) / 8, sm_count() * 16));
+    const int g2 = (int)std::max<int64_t>(1, std::min<int64_t>((kept + 255) / 256, sm_count() * 16));
     if (d->dtype == VBG_C128)
       gather_blocks_kernel<cplx><<<g2, 256, 0, s>>>(kept, old_of.as<int>(), m->blk_off.as<int64_t>(),
                                                     m->vals.as<cplx>(), d->blk_off.as<int64_t>(), d->vals.as<cplx>());
