@@ -337,15 +337,33 @@ py::array_t<T> to_array(const std::vector<T>& v) {
 }
 
 // ---------------------------------------------------------------- matrix
+// The graph of a matrix, read back from the device when it is first asked
+// for: a product's structure is built on the device, and a chain of products,
+// sums and filters never looks at it on the host (reading it after each cost
+// 1.5-3 ms of the 11 ms of a product with 500k blocks).
+struct LazyGraph {
+  mutable GraphPtr p;
+  const vbg_matrix* src = nullptr;  // whose structure p is, while p is unset
+  LazyGraph(GraphPtr g) : p(std::move(g)) {}
+  explicit LazyGraph(const vbg_matrix* m) : src(m) {}
+  const GraphPtr& get() const {
+    if (!p) p = graph_from_device(src);
+    return p;
+  }
+  Graph* operator->() const { return get().get(); }
+  Graph& operator*() const { return *get(); }
+  operator GraphPtr() const { return get(); }
+};
+
 template <typename T>
 struct Mat {
-  GraphPtr g;
+  LazyGraph g;
   std::vector<T> host;
   bool host_ok = true, dev_ok = false;
   vbg_matrix* dm = nullptr;
 
   explicit Mat(GraphPtr gr) : g(std::move(gr)) { host.assign(g->nnz(), T(0)); }
-  Mat(GraphPtr gr, int) : g(std::move(gr)) {}
+  Mat(LazyGraph gr, int) : g(std::move(gr)) {}
   Mat(const Mat&) = delete;
   ~Mat() {
     if (dm) vbg_matrix_destroy(dm);
@@ -364,9 +382,22 @@ struct Mat {
       dev_ok = true;
     }
   }
+  // Sizes without the graph's lists where the device matrix has them.
+  struct Sizes {
+    int kind = 0;
+    int64_t nnzb = 0, nnz = 0, N = 0;
+  };
+  Sizes sizes() const {
+    Sizes z;
+    check(vbg_matrix_info(dm, nullptr, nullptr, &z.nnzb, &z.nnz, &z.N, &z.kind), "vbg_matrix_info");
+    return z;
+  }
+  int64_t N() const { return dm ? sizes().N : g->N(); }
+  int64_t nnz() const { return dm ? sizes().nnz : g->nnz(); }
+  int64_t nnzb() const { return dm ? sizes().nnzb : g->nnzb(); }
   void ensure_host() {
     if (host_ok) return;
-    host.resize(g->nnz());
+    host.resize(nnz());
     check(vbg_matrix_get_values(dm, host.data(), stream()), "vbg_matrix_get_values");
     host_ok = true;
   }
@@ -374,22 +405,23 @@ struct Mat {
   void host_modified() { dev_ok = false; }
   // After an operation that may have changed the device pattern.
   void adopt_device_structure() {
-    int n = 0;
-    int64_t nnzb = 0;
-    check(vbg_matrix_info(dm, nullptr, &n, &nnzb, nullptr, nullptr, nullptr), "vbg_matrix_info");
-    bool same = nnzb == g->nnzb();
-    if (same) {
-      std::vector<int> rp(n + 1), ci(std::max<int64_t>(nnzb, 1));
-      check(vbg_matrix_get_structure(dm, rp.data(), ci.data(), nullptr), "vbg_matrix_get_structure");
-      ci.resize(nnzb);
-      same = rp == g->row_ptr && ci == g->col_ind;
+    if (g.p) {  // the same object while the pattern is the same
+      const int n = g->n;
+      const int64_t nb = nnzb();
+      bool same = nb == g->nnzb();
+      if (same) {
+        std::vector<int> rp(n + 1), ci(std::max<int64_t>(nb, 1));
+        check(vbg_matrix_get_structure(dm, rp.data(), ci.data(), nullptr), "vbg_matrix_get_structure");
+        ci.resize(nb);
+        same = rp == g->row_ptr && ci == g->col_ind;
+      }
+      if (!same) g = LazyGraph(dm);
     }
-    if (!same) g = graph_from_device(dm);
     host_ok = false;
     dev_ok = true;
   }
   static std::unique_ptr<Mat> wrap_device(vbg_matrix* d) {
-    auto m = std::unique_ptr<Mat>(new Mat(graph_from_device(d), 0));
+    auto m = std::unique_ptr<Mat>(new Mat(LazyGraph(d), 0));
     m->dm = d;
     m->host_ok = false;
     m->dev_ok = true;
@@ -508,7 +540,7 @@ void bind_matrix(py::module& m, const char* name) {
   };
   py::class_<M>(m, name)
       .def(py::init([](GraphPtr g) { return std::make_unique<M>(g); }), py::keep_alive<1, 2>())
-      .def_property_readonly("graph", [](const M& a) { return a.g; })
+      .def_property_readonly("graph", [](const M& a) { return a.g.get(); })
       .def("add_block", &M::add_block, py::arg("g_row"), py::arg("g_col"), py::arg("data"),
            py::arg("mode") = AssemblyMode::ADD)
       .def("set_values", &M::set_values, py::arg("values"))
@@ -530,7 +562,7 @@ void bind_matrix(py::module& m, const char* name) {
         a.device_modified();
       })
       .def("add_diagonal", [](M& a, SV& v) {
-        if (v.rows < a.g->N()) throw std::runtime_error("Vector size too small for add_diagonal");
+        if (v.rows < a.N()) throw std::runtime_error("Vector size too small for add_diagonal");
         a.ensure_device();
         check(vbg_matrix_add_diagonal(a.dm, v.read(), stream()), "add_diagonal");
         a.device_modified();
@@ -582,16 +614,16 @@ void bind_matrix(py::module& m, const char* name) {
         a.host_modified();
       })
       .def("duplicate", [](M& a, bool independent_graph) {
-        auto g = independent_graph ? std::make_shared<Graph>(*a.g) : a.g;
-        auto d = std::make_unique<M>(g, 0);
         if (a.dev_ok && a.dm) {
-          check(vbg_matrix_duplicate(a.dm, &d->dm, stream()), "duplicate");
-          d->dev_ok = true;
-          d->host_ok = false;
-        } else {
-          d->host = a.host;
-          d->host_ok = true;
+          vbg_matrix* dm = nullptr;
+          check(vbg_matrix_duplicate(a.dm, &dm, stream()), "duplicate");
+          auto d = M::wrap_device(dm);
+          if (!independent_graph) d->g = a.g.get();
+          return d;
         }
+        auto d = std::make_unique<M>(LazyGraph(independent_graph ? std::make_shared<Graph>(*a.g) : a.g.get()), 0);
+        d->host = a.host;
+        d->host_ok = true;
         return d;
       }, py::arg("independent_graph") = true)
       .def("spmm", [](M& a, M& b, double thr, bool transA, bool transB) {
@@ -644,14 +676,14 @@ void bind_matrix(py::module& m, const char* name) {
       })
       .def("real", [](M& a) {
         a.ensure_host();
-        auto r = std::make_unique<MatD>(a.g);
+        auto r = std::make_unique<MatD>(a.g.get());
         for (size_t i = 0; i < a.host.size(); ++i) r->host[i] = cplx(a.host[i]).real();
         r->host_modified();
         return r;
       })
       .def("imag", [](M& a) {
         a.ensure_host();
-        auto r = std::make_unique<MatD>(a.g);
+        auto r = std::make_unique<MatD>(a.g.get());
         for (size_t i = 0; i < a.host.size(); ++i) r->host[i] = cplx(a.host[i]).imag();
         r->host_modified();
         return r;
@@ -664,7 +696,7 @@ void bind_matrix(py::module& m, const char* name) {
       })
       .def("get_block_density", [](const M& a) {
         const double n = a.g->n;
-        return n == 0 ? 0.0 : (double)a.g->nnzb() / (n * n);
+        return n == 0 ? 0.0 : (double)a.nnzb() / (n * n);
       })
       .def("get_block", [](M& a, int row, int col) {
         if (row < 0 || row >= a.g->n || col < 0 || col >= a.g->n) return py::array_t<T>();
@@ -677,8 +709,12 @@ void bind_matrix(py::module& m, const char* name) {
         return out;
       }, py::arg("row"), py::arg("col"))
       .def("get_values", [](M& a) {
-        a.ensure_host();
-        return to_array(a.host);
+        if (a.host_ok) return to_array(a.host);
+        // straight into the result (the host copy is left for those who
+        // change it: filling it first and copying it took 84 ms for 144 MB)
+        py::array_t<T> out((py::ssize_t)a.nnz());
+        if (out.size()) check(vbg_matrix_get_values(a.dm, out.mutable_data(), stream()), "vbg_matrix_get_values");
+        return out;
       })
       .def("to_dense", [](M& a) {
         a.ensure_host();
@@ -758,13 +794,13 @@ void bind_matrix(py::module& m, const char* name) {
         }
         return std::string(mx <= 1 ? "csr" : (mn == mx ? "bsr" : "vbcsr"));
       })
-      .def_property_readonly("local_nnz", [](const M& a) { return a.g->nnz(); })
-      .def_property_readonly("global_nnz", [](const M& a) { return a.g->nnz(); })
-      .def_property_readonly("local_block_nnz", [](const M& a) { return a.g->nnzb(); })
-      .def_property_readonly("owned_scalar_rows", [](const M& a) { return a.g->N(); })
-      .def_property_readonly("global_scalar_rows", [](const M& a) { return a.g->N(); })
-      .def_property_readonly("global_scalar_cols", [](const M& a) { return a.g->N(); })
-      .def_property_readonly("shape", [](const M& a) { return py::make_tuple(a.g->N(), a.g->N()); })
+      .def_property_readonly("local_nnz", [](const M& a) { return a.nnz(); })
+      .def_property_readonly("global_nnz", [](const M& a) { return a.nnz(); })
+      .def_property_readonly("local_block_nnz", [](const M& a) { return a.nnzb(); })
+      .def_property_readonly("owned_scalar_rows", [](const M& a) { return a.N(); })
+      .def_property_readonly("global_scalar_rows", [](const M& a) { return a.N(); })
+      .def_property_readonly("global_scalar_cols", [](const M& a) { return a.N(); })
+      .def_property_readonly("shape", [](const M& a) { return py::make_tuple(a.N(), a.N()); })
       .def_property_readonly("row_ptr", [](const M& a) { return to_array(a.g->row_ptr); })
       .def_property_readonly("col_ind", [](const M& a) { return to_array(a.g->col_ind); })
       .def_property_readonly("configured_page_size", [](const M&) { return 0; })

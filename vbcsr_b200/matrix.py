@@ -60,15 +60,25 @@ class VBCSR(LinearOperator):
     def _wrap_core(cls, core: Any, dtype, comm: Any, shape: Optional[Tuple[int, int]] = None,
                    global_nnz: Optional[int] = None) -> "VBCSR":
         obj = cls.__new__(cls)
-        obj.graph = core.graph
+        obj._graph = None  # read from the core when first asked for
         obj.dtype = np.dtype(dtype)
         obj.comm = comm
         obj._core = core
         obj.shape = shape if shape is not None else tuple(int(s) for s in core.shape)
         return obj
 
+    @property
+    def graph(self) -> Any:
+        if self._graph is None:
+            self._graph = self._core.graph
+        return self._graph
+
+    @graph.setter
+    def graph(self, value: Any) -> None:
+        self._graph = value
+
     def _refresh_graph(self) -> None:
-        self.graph = self._core.graph
+        self._graph = None
 
     # ---- properties (matrix.py:99-250) ----
     @property
@@ -138,7 +148,7 @@ class VBCSR(LinearOperator):
 
     def transpose_(self) -> None:
         self._core = self._core.transpose()
-        self.graph = self._core.graph
+        self._refresh_graph()
         self.shape = (self.shape[1], self.shape[0])
 
     def conj_(self) -> None:
