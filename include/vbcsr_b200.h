@@ -213,6 +213,22 @@ int vbg_cheb_step_adjoint(const vbg_matrix* m, int k, int ld, double alpha, doub
 int vbg_cheb_series(const vbg_matrix* m, int k, int ld, const void* V, int M, const double* coeffs, double scale,
                     double center, void* psi, int K, void* ckpt, void* stream);
 
+/* `steps` steps of a vector recurrence with its vectors as columns (no
+ * counterpart in the reference, which has no gradients):
+ *     y_s = alpha_s B y_{s-1} + beta_s y_{s-1} + gamma_s y_{s-2} + c_s g
+ * with B = A or (adjoint != 0) A^H, y_{-1} = x0, y_{-2} = x1 (NULL: zero) and
+ * g = source (NULL: none).  coeffs: HOST array of {alpha, beta, gamma, re c,
+ * im c} per step.  With cols != NULL, x0 is written to column col0 of the
+ * row-major N x ncol matrix cols (leading dimension ldc) and y_s to column
+ * col0 + (s + 1) dcol, columns outside [0, ncol) being skipped: the
+ * multivectors of vbg_sddmm.  last / before (may be NULL) receive the last
+ * vector and the one before it.  One launch for all steps when the matrix
+ * fits the SMs' shared memory (its values at most about 30 MB, blocks at most
+ * 8 x 8), as vbg_cheb_series does for vectors. */
+int vbg_cheb_columns(const vbg_matrix* m, int adjoint, const void* x0, const void* x1, int steps,
+                     const double* coeffs, const void* source, void* cols, int64_t ldc, int ncol, int col0, int dcol,
+                     void* last, void* before, void* stream);
+
 /* vbg_cheb_step with dots, for callers that cannot let the library allocate
  * device memory (no counterpart in the reference).  vbg_cheb_step allocates
  * its per-CTA reduction scratch on first use; this variant allocates nothing

@@ -80,6 +80,7 @@ _SIGNATURES = {
     "vbg_matrix_norm_fro": ([_vp, _vp, _vp], _i),
     "vbg_sddmm": ([_vp, _i, _i, _vp, _vp, _d, _d, _vp, _vp], _i),
     "vbg_cheb_series": ([_vp, _i, _i, _vp, _i, _vp, _d, _d, _vp, _i, _vp, _vp], _i),
+    "vbg_cheb_columns": ([_vp, _i, _vp, _vp, _i, _vp, _vp, _vp, C.c_int64, _i, _i, _i, _vp, _vp, _vp], _i),
     "vbg_apply_tile_rows": ([_vp, _i, _i, _pi], _i),
     "vbg_matrix_create_device": ([C.POINTER(_vp), _i, _i, _vp, C.c_int64, _vp, _vp, _vp, _vp], _i),
     "vbg_square_polynomial_upper": ([_vp, _d, _d, _d, _d, _d, _d, _d, C.POINTER(_vp), _vp], _i),

@@ -206,9 +206,60 @@ def _cheb_series(op, scale, center, v, coeffs, K):
     return psi, None, ckpt
 
 
-def _cheb_backward(op, scale, center, v, M, K, ckpt, source):
-    """Adjoint recurrence; returns (dL/dH~* on the pattern as a value array,
-    a_0).  source(n) -> s_n (tensor shaped like v, or None)."""
+def _cheb_columns(op, adjoint, x0, x1, coeffs, source, cols, col0, dcol, last=None, before=None):
+    """vbg_cheb_columns: len(coeffs) steps from x0, x1 into the columns of cols."""
+    c = np.ascontiguousarray(coeffs, dtype=np.float64)
+    opt = lambda t: _ptr(t) if t is not None else None  # noqa: E731
+    _capi.call("vbg_cheb_columns", op.h, int(adjoint), _ptr(x0), opt(x1), len(c), c.ctypes.data_as(_vp), opt(source),
+               _ptr(cols), cols.stride(0), cols.shape[1], col0, dcol, opt(last), opt(before), _stream())
+
+
+def _cheb_backward_vector(op, scale, center, v, M, K, ckpt, src, src_coef):
+    """_cheb_backward for a plain vector, s_n = src_coef[n] src: the t's and
+    the a's of a segment are each one vbg_cheb_columns call that writes them
+    as the columns the SDDMM reads."""
+    dH = torch.zeros(op.nnz, dtype=v.dtype if v.is_complex() else torch.float64, device=v.device)
+    center = float(np.real(center))
+    sc = np.asarray(src_coef, dtype=np.complex128)
+    src = src.contiguous()
+    a1 = src * (complex(sc[M - 1]) if v.is_complex() else float(sc[M - 1].real))  # a_{M-1}
+    a2 = None
+    for s0 in reversed(range(0, M, K)):
+        w = min(s0 + K, M - 1) - s0  # the pairs (a_{n+1}, t_n) of n = s0 .. s0 + w - 1
+        if w <= 0:
+            continue
+        T = torch.empty((v.shape[0], w), dtype=v.dtype, device=v.device)
+        G = torch.empty_like(T)
+        t, t_prev = ckpt[s0]
+        n = s0 + 1 + np.arange(w - 1)
+        wt = np.where(n == 1, 1.0, 2.0)
+        zero = np.zeros(len(n))
+        _cheb_columns(op, False, t, t_prev, np.stack([wt / scale, -wt * center / scale, np.where(n == 1, 0.0, -1.0),
+                                                      zero, zero], axis=1), None, T, 0, 1)
+        n = s0 + w - 1 - np.arange(w)  # a_n = s_n + w_n H~^H a_{n+1} - a_{n+2}
+        wt = np.where(n == 0, 1.0, 2.0)
+        gamma = np.full(w, -1.0)
+        if a2 is None:
+            gamma[0] = 0.0
+        last, before = torch.empty_like(v), torch.empty_like(v)
+        _cheb_columns(op, True, a1, a2, np.stack([wt / scale, -wt * center / scale, gamma, sc.real[n], sc.imag[n]],
+                                                 axis=1), src, G, w - 1, -1, last, before)
+        if s0 == 0:
+            G[:, 0] *= 0.5  # n = 0 has weight 1; the SDDMM's alpha is 2
+        _sddmm(op, G, T, dH, alpha=2.0)
+        a1, a2 = last, before
+    return dH / scale, a1
+
+
+def _cheb_backward(op, scale, center, v, M, K, ckpt, src, src_coef):
+    """Adjoint recurrence with sources s_n = src_coef[n] src; returns (dL/dH~*
+    on the pattern as a value array, a_0)."""
+    if v.dim() == 1:
+        return _cheb_backward_vector(op, scale, center, v, M, K, ckpt, src, src_coef)
+
+    def source(n):
+        return None if src_coef[n] == 0.0 else src * src_coef[n]
+
     dH = torch.zeros(op.nnz, dtype=v.dtype if v.is_complex() else torch.float64, device=v.device)
     a1 = a2 = None  # a_{n+1}, a_{n+2}
     scratch = torch.empty_like(v) if v.dim() == 1 else torch.empty(v.shape[0], v.stride(0), dtype=v.dtype,
@@ -261,12 +312,8 @@ class ChebyshevPropagation(torch.autograd.Function):
         op = ctx.op
         _set_values(op, values)
         coeffs = ctx.coeffs
-        g = _padded(g)
-
-        def source(n):
-            return g * np.conj(coeffs[n])
-
-        dH, a0 = _cheb_backward(op, ctx.scale, ctx.center, _padded(psi0), len(coeffs), ctx.K, ctx.ckpt, source)
+        dH, a0 = _cheb_backward(op, ctx.scale, ctx.center, _padded(psi0), len(coeffs), ctx.K, ctx.ckpt, _padded(g),
+                                np.conj(coeffs))
         ctx.ckpt = None
         gV = dH if ctx.needs_input_grad[0] else None
         gpsi = a0 if ctx.needs_input_grad[1] else None
@@ -309,13 +356,10 @@ class KPMMoments(torch.autograd.Function):
         op = ctx.op
         _set_values(op, values)
         Vp = _padded(V)
-        gm = gmu.detach().cpu().numpy()
-
-        def source(n):
-            # mu_0 = <v, v> does not depend on H; mu_n = <v, t_n> for n >= 1
-            return None if n == 0 or gm[n] == 0.0 else Vp * float(gm[n])
-
-        dH, _ = _cheb_backward(op, ctx.scale, ctx.center, Vp, ctx.M, ctx.K, ctx.ckpt, source)
+        # mu_0 = <v, v> does not depend on H; mu_n = <v, t_n> for n >= 1
+        gm = gmu.detach().cpu().numpy().copy()
+        gm[0] = 0.0
+        dH, _ = _cheb_backward(op, ctx.scale, ctx.center, Vp, ctx.M, ctx.K, ctx.ckpt, Vp, gm)
         ctx.ckpt = None
         return (dH if ctx.needs_input_grad[0] else None), None, None, None, None, None, None
 

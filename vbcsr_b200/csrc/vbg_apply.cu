@@ -523,6 +523,7 @@ __global__ void __launch_bounds__(kThreads) apply_mv_kernel(ApplyArgs a, const T
 #include "vbg_pipe.cuh"
 #include "vbg_tile.cuh"
 #include "vbg_chain.cuh"
+#include "vbg_resident.cuh"
 // Forward vectors on matrices whose blocks are all at most 8 x 8, every row
 // from the slot records (vec_row_meta): a kernel of its own so that its
 // register budget is not set by the general row paths: with 36 warps per
@@ -1980,6 +1981,35 @@ int vbg_cheb_series(const vbg_matrix* m, int k, int ld, const void* V, int M, co
   VBG_CUDA(cudaMemsetAsync(psi, 0, bytes, s));
   if ((rc = vbg_mv_axpby(dtype, rows, k, ld, coeffs[0], coeffs[1], V, 0.0, 0.0, psi, stream))) return rc;
   if (M == 1) return 0;
+  if (ld == 1 && !g_opt_vec_kernel.load()) {
+    // the whole series in one launch when the matrix fits the SMs' shared memory
+    std::vector<double> cf((size_t)(M - 1) * kResCoef);
+    for (int n = 1; n < M; ++n) {
+      const double w = n == 1 ? 1.0 : 2.0;
+      double* c = &cf[(size_t)(n - 1) * kResCoef];
+      c[0] = w / scale;
+      c[1] = -w * center / scale;
+      c[2] = n == 1 ? 0.0 : -1.0;
+      c[3] = coeffs[2 * n];
+      c[4] = coeffs[2 * n + 1];
+    }
+    ResidentArgs a{};
+    a.x0 = V;
+    a.steps = M - 1;
+    a.psi = psi;
+    a.K = K;
+    a.M = M;
+    a.ckpt = ckpt;
+    DevBuf scratch(s);
+    bool ran = false;
+    if ((rc = resident_run(m, false, a, cf.data(), scratch, s, &ran))) return rc;
+    if (ran) {
+      // K = 1: the first pair's t_0 is V
+      if (K == 1)
+        VBG_CUDA(cudaMemcpyAsync(static_cast<char*>(ckpt) + bytes, V, bytes, cudaMemcpyDeviceToDevice, s));
+      return 0;
+    }
+  }
   DevBuf buf[3] = {DevBuf(s), DevBuf(s), DevBuf(s)};
   for (auto& b : buf) {
     if ((rc = b.ensure(std::max<size_t>(bytes, 16)))) return rc;
@@ -2019,6 +2049,66 @@ int vbg_cheb_series(const vbg_matrix* m, int k, int ld, const void* V, int M, co
     t = y;
   }
   return 0;
+}
+
+int vbg_cheb_columns(const vbg_matrix* m, int adjoint, const void* x0, const void* x1, int steps,
+                     const double* coeffs, const void* source, void* cols, int64_t ldc, int ncol, int col0, int dcol,
+                     void* last, void* before, void* stream) {
+  VBG_CHECK(m && x0 && coeffs, VBG_E_ARG, "null argument");
+  VBG_CHECK(steps >= 0 && (!cols || (ncol >= 0 && ldc >= ncol)), VBG_E_ARG, "invalid steps / ncol / ldc");
+  cudaStream_t s = as_stream(stream);
+  if (m->N == 0) return 0;
+  const size_t es = elem_size(m->dtype), bytes = (size_t)m->N * es;
+  int rc;
+  auto copy = [&](void* to, const void* from) -> int {
+    if (to && to != from) VBG_CUDA(cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToDevice, s));
+    return 0;
+  };
+  auto column = [&](int c, const void* v) -> int {
+    if (cols && c >= 0 && c < ncol)
+      VBG_CUDA(cudaMemcpy2DAsync(static_cast<char*>(cols) + (size_t)c * es, (size_t)ldc * es, v, es, es, m->N,
+                                 cudaMemcpyDeviceToDevice, s));
+    return 0;
+  };
+  ResidentArgs a{};
+  a.x0 = x0;
+  a.x1 = x1;
+  a.steps = steps;
+  a.source = source;
+  a.cols = cols;
+  a.ldc = ldc;
+  a.col0 = col0;
+  a.dcol = dcol;
+  a.ncol = ncol;
+  DevBuf scratch(s);
+  bool ran = false;
+  // (a forced vector kernel runs its own steps)
+  if (!g_opt_vec_kernel.load() && (rc = resident_run(m, adjoint != 0, a, coeffs, scratch, s, &ran))) return rc;
+  if (ran) {
+    if ((rc = copy(last, a.xch[(steps - 1) & 1]))) return rc;
+    return copy(before, steps > 1 ? a.xch[steps & 1] : x0);
+  }
+  // a fused step at a time, on three working vectors
+  if ((rc = column(col0, x0))) return rc;
+  DevBuf buf(s);
+  const size_t room = (bytes + 255) / 256 * 256;
+  if ((rc = buf.ensure(3 * room))) return rc;
+  const void *x = x0, *p = x1;
+  for (int k = 0; k < steps; ++k) {
+    const double* c = coeffs + (size_t)kResCoef * k;
+    char* y = buf.as<char>();
+    while (y == x || y == p) y += room;
+    const double gamma = p ? c[2] : 0.0;
+    if ((rc = fused_step(m, adjoint != 0, 1, 1, c[0], c[1], gamma, x, p, y, nullptr, nullptr, nullptr, 0.0, 0.0,
+                         stream)))
+      return rc;
+    if (source && (rc = vbg_mv_axpby(m->dtype, m->N, 1, 1, c[3], c[4], source, 1.0, 0.0, y, stream))) return rc;
+    if ((rc = column(col0 + (k + 1) * dcol, y))) return rc;
+    p = x;
+    x = y;
+  }
+  if ((rc = copy(last, x))) return rc;
+  return p ? copy(before, p) : 0;
 }
 
 int vbg_kpm_moments(const vbg_matrix* m, int R, int ld, const void* V0, int M, int precision, int two_moment,

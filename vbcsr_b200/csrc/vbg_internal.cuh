@@ -219,6 +219,14 @@ struct ChainPlan {
   DevBuf qidx, rowinfo;  // as TilePlan's, in cache rows
 };
 
+// Block rows per CTA of the shared-memory-resident vector recurrence
+// (vbg_resident.cuh); grid 0: the matrix does not fit.
+struct ResidentPlan {
+  int grid = 0;
+  size_t smem = 0;
+  DevBuf cta, rows, xlist, place;
+};
+
 // CUDA-graph cache entry for a replayable recurrence.
 struct GraphEntry {
   cudaGraph_t graph = nullptr;
@@ -306,6 +314,8 @@ struct vbg_matrix {
   std::map<std::pair<int, int>, int> tile_queue;
   // Chained row tiles (vbg_chain.cuh), per (X row bytes, value scalar size).
   std::map<std::pair<int, int>, std::unique_ptr<vbg::ChainPlan>> chain_plans;
+  // Resident vector recurrences, [0] over the rows, [1] over the columns.
+  std::unique_ptr<vbg::ResidentPlan> resident[2];
   // The autotuner's choice of forward multivector kernel (VBG_KERNEL_*) per
   // (leading dimension, FP32 values).
   std::map<std::pair<int, int>, int> tuned;
@@ -341,6 +351,8 @@ struct vbg_matrix {
     tile_rows_cap.clear();
     tile_queue.clear();
     chain_plans.clear();
+    resident[0].reset();
+    resident[1].reset();
     tuned.clear();
     invalidate_values();
   }
