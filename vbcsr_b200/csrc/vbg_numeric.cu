@@ -171,9 +171,19 @@ __device__ __forceinline__ void pair_mma(cplx (&acc)[2], cplx a, cplx b) {
 __device__ __forceinline__ double sq_abs(double v) { return __dmul_rn(v, v); }
 __device__ __forceinline__ double sq_abs(cplx v) { return fma(v.re, v.re, __dmul_rn(v.im, v.im)); }
 
+// CTAs per SM and pairs in flight of the sparse form.  It is bound by the
+// latency of its short loops, so warps count for more than pairs in flight:
+// for whole products of 12000 rows (real) and a 60 x 60 lattice (complex),
+// two CTAs of four or two pairs took 2272 and 1173 us, three of two 1952,
+// four of one 1072.
+template <typename T>
+constexpr int kSparseCtas = std::is_same<T, cplx>::value ? 4 : 3;
+template <typename T>
+constexpr int kSparsePairs = std::is_same<T, cplx>::value ? 1 : 2;
+
 template <typename T, bool GATED, bool DENSE>
-__global__ void __launch_bounds__(512, 1) numeric_pairs_kernel(PairsArgs a, const T* __restrict__ A,
-                                                               const T* __restrict__ B, T* __restrict__ C) {
+__global__ void __launch_bounds__(DENSE ? 512 : 256, DENSE ? 1 : kSparseCtas<T>)
+    numeric_pairs_kernel(PairsArgs a, const T* __restrict__ A, const T* __restrict__ B, T* __restrict__ C) {
   constexpr int J = PairsJ<T>::v;
   extern __shared__ __align__(16) unsigned char pairs_raw[];
   __shared__ short wtab[kWin];
@@ -401,7 +411,7 @@ __global__ void __launch_bounds__(512, 1) numeric_pairs_kernel(PairsArgs a, cons
           const unsigned m = kb + lane < nk ? (unsigned)bits[kb + lane] >> c : 0u;
           const unsigned w0 = __ballot_sync(0xffffffffu, m & 1u), w1 = __ballot_sync(0xffffffffu, m & 16u);
           for (unsigned w = w0 | w1; w;) {
-            constexpr int U = std::is_same<T, cplx>::value ? 2 : 4;
+            constexpr int U = kSparsePairs<T>;
             T fa0[U][2], fa1[U][2], fb[U][2];
             int in[U];
             unsigned at[U];
@@ -492,11 +502,17 @@ int numeric_pairs(const vbg_matrix* A, const vbg_matrix* B, vbg_matrix* C, const
   // offsets into B and indexes into the list are 32 and 16 bits wide
   if (B->nnz >= (int64_t)INT32_MAX || kc > 32767 || max_vals == INT32_MAX) return kNumericNotFit;
   const size_t fixed = kWin * sizeof(short) + 1024;  // the window table and the system's share
-  // eight warps and two CTAs per SM, else sixteen warps and one
+  // the sparse form runs eight warps, the dense one eight with two CTAs per SM,
+  // else (also where the sparse form's do not fit) sixteen with one
+  bool dense = pairs * A->n >= kDenseShare * (double)C->nnzb * (double)A->nnzb;
   int warps = 8;
-  if (pairs_smem(kc, max_vals, es, J, 8) + fixed > kPairsSmem2) warps = 16;
-  const size_t smem = pairs_smem(kc, max_vals, es, J, warps);
-  if (smem + fixed > kPairsSmem1) return kNumericNotFit;
+  size_t smem = pairs_smem(kc, max_vals, es, J, warps);
+  if (smem + fixed > (dense ? kPairsSmem2 : kPairsSmem1)) {
+    dense = true;
+    warps = 16;
+    smem = pairs_smem(kc, max_vals, es, J, warps);
+    if (smem + fixed > kPairsSmem1) return kNumericNotFit;
+  }
   RowPairs cj(s);
   int rc;
   if (!A->n) return 0;
@@ -531,7 +547,6 @@ int numeric_pairs(const vbg_matrix* A, const vbg_matrix* B, vbg_matrix* C, const
   a.kc = kc;
   a.vc = max_vals;
   const bool gated = gate.mode != kGateSum || gate.bound_out || !gate.drop;
-  const bool dense = pairs * A->n >= kDenseShare * (double)C->nnzb * (double)A->nnzb;
   return cx ? launch_pairs<cplx>(a, gated, dense, warps, smem, A, B, C, s)
             : launch_pairs<double>(a, gated, dense, warps, smem, A, B, C, s);
 }
