@@ -76,9 +76,11 @@ int vbg_device_status(unsigned* status, int clear);
  *   "apply.autotune" 1 (default): the first forward multivector apply with a
  *                  given leading dimension and precision on a matrix (outside
  *                  stream capture; vbg_kpm_moments* before their capture)
- *                  times the kernels that can run it -- chained tiles, tiles,
- *                  pipelined -- and keeps the fastest for that matrix; the
- *                  trials overwrite Y and the dots, never the accumulator.
+ *                  chooses its kernel: by the structure and sizes where
+ *                  kernels add in different orders, by timing between the
+ *                  ones that add alike (tiles and chained tiles at 512-byte
+ *                  rows, FP32 at 64 columns and up); the trials overwrite Y
+ *                  and the dots, never the accumulator.
  *                  0: the default order (chained tiles for FP32 only).
  *                  vbg_apply_kernel reports the tuned choice once made.
  * An unknown name returns VBG_E_ARG.  Graphs captured before a change keep
@@ -155,7 +157,7 @@ int vbg_spmm(const vbg_matrix* m, int k, int ld, const void* X, void* Y, void* s
  * 16-byte-aligned buffers (no counterpart in the reference).  Builds the
  * value layout and tile plan that choice needs, as the first apply would. */
 #define VBG_KERNEL_VECTOR 0 /* ld == 1: a warp per block row, lanes over (block, row) pairs */
-#define VBG_KERNEL_ROWS 1   /* a warp per block row, X rows read per lane */
+#define VBG_KERNEL_ROWS 1   /* warps per block row, X rows read from memory (FP64, complex: tensor cores) */
 #define VBG_KERNEL_PIPE 2   /* a warp per block row, spans staged by bulk copies */
 #define VBG_KERNEL_TILE 3   /* a CTA per tile of block rows, X ranges staged once per tile */
 #define VBG_KERNEL_CHAIN 4  /* tiles chained per persistent CTA, X rows cached across tiles */
@@ -163,7 +165,7 @@ int vbg_spmm(const vbg_matrix* m, int k, int ld, const void* X, void* Y, void* s
 int vbg_apply_kernel(const vbg_matrix* m, int ld, int precision, int* kernel);
 /* Block rows per tile of the tiled kernel's plan for applies at this leading
  * dimension and precision (no counterpart in the reference): the height the
- * autotuner kept (it times tiles of at most 16, 12 and 8 block rows), or the
+ * autotuner kept (of tiles of at most 16, 12 and 8 block rows), or the
  * tallest that fits before it has run; 0 when no tile plan exists yet. */
 int vbg_apply_tile_rows(const vbg_matrix* m, int ld, int precision, int* rows);
 /* Y = A^H X.  block_csr.hpp:1038 mult_dense_adjoint. */

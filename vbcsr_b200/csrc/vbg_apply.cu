@@ -522,6 +522,7 @@ __global__ void __launch_bounds__(kThreads) apply_mv_kernel(ApplyArgs a, const T
 // ------------------------------------------------ pipelined multivector apply
 #include "vbg_pipe.cuh"
 #include "vbg_tile.cuh"
+#include "vbg_dtile.cuh"
 #include "vbg_chain.cuh"
 #include "vbg_resident.cuh"
 // Forward vectors on matrices whose blocks are all at most 8 x 8, every row
@@ -1159,13 +1160,6 @@ static int launch_pipe_t(const vbg_matrix* m, const ApplyArgs& a, cudaStream_t s
   }
 }
 
-// Whether this apply runs on apply_tile_kernel<T, EV, G>: a row of X is
-// 32 / G lanes of EV scalars (ld = 32 / G * EV: FP64 and FP32 at 64
-// columns with EV = 2, complex and FP32 at 32 with EV = 1, FP64 and FP32 at
-// 16 with EV = 1 and G = 2 lane groups), the pipelined apply's value layout
-// applies, the bulk-copied rows (X, Xprev, the dot partner) start on 16-byte
-// boundaries, and the matrix has a tile plan for it (built here unless
-// capturing or allocation is not allowed).
 // Largest tile height (block rows) of the tiled applies at this leading
 // dimension and value size: the autotuner's choice, kTileRowsMax before it.
 static int tile_cap(const vbg_matrix* m, int ld, int es) {
@@ -1180,15 +1174,35 @@ static bool tile_queue_on(const vbg_matrix* m, int ld, int es) {
   return it != m->tile_queue.end() && it->second != 0;
 }
 
+// Pieces of 128 bytes of a multivector row with leading dimension ld that
+// apply_dtile_kernel<T, NP> takes (1 or 2), else 0.  At four pieces the
+// tensor pipe (blocks of 3 and 5 fill 3 and 5 eighths of a step) is the
+// bound, and scalar multiply-adds with two columns a lane are faster: 200 x
+// 200 lattice, FP64, 64 columns: 410 us a step against 313.
+template <typename T>
+static int dtile_pieces(int ld) {
+  const int64_t bytes = (int64_t)ld * (int)sizeof(T);
+  return std::is_same<T, float>::value || (bytes != 128 && bytes != 256) ? 0 : (int)(bytes / 128);
+}
+
+// Whether this apply runs on a tiled kernel: FP64 and complex on
+// apply_dtile_kernel<T, NP> when a row of X is 1 or 2 pieces of 128 bytes,
+// else on apply_tile_kernel<T, EV, G> when it is 32 / G lanes of EV scalars
+// (FP64 and FP32 at 64 columns, complex at 32; FP32 at 32 and 16 columns
+// with EV = 4 and G = 4 and 8 lane groups); the pipelined apply's value
+// layout applies, the staged rows (X, Xprev, the dot partner) start on
+// 16-byte boundaries, and the matrix has a tile plan for it (built here
+// unless capturing or allocation is not allowed).
 template <typename T, int EV = PipeEV<T>::v, int G = 1>
 static bool tile_use(const vbg_matrix* m, bool adj, const ApplyArgs& a, cudaStream_t s, bool allow_alloc,
                      TilePlan** plan) {
   *plan = nullptr;
-  if (a.ld != 32 / G * EV || !pipe_use<T>(m, adj, a, s, allow_alloc)) return false;
+  if (dtile_pieces<T>(a.ld) == 0 && a.ld != 32 / G * EV) return false;
+  if (!pipe_use<T>(m, adj, a, s, allow_alloc)) return false;
   const void* copied[3] = {a.X, a.Xprev, a.dotw};
   for (const void* p : copied)
     if (p && reinterpret_cast<uintptr_t>(p) % 16) return false;
-  const int rb = 32 / G * EV * (int)sizeof(T);
+  const int rb = a.ld * (int)sizeof(T);
   const int cap = tile_cap(m, a.ld, (int)sizeof(T));
   auto it = m->tile_plans.find(std::make_tuple(rb, (int)sizeof(T), cap));
   if (it != m->tile_plans.end()) {
@@ -1208,13 +1222,13 @@ static int tile_grid(TilePlan* plan, int* grid) {
   static bool attr_set[kMaxDevices] = {};
   const int dev = current_device();
   if (!attr_set[dev]) {
-    VBG_CUDA(cudaFuncSetAttribute(apply_tile_kernel<T, EV, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    VBG_CUDA(cudaFuncSetAttribute(apply_tile_kernel<T, EV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)kTileSmemBudget));
     attr_set[dev] = true;
   }
   if (!plan->grid) {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, apply_tile_kernel<T, EV, G>, kTileWarps * 32, plan->smem) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, apply_tile_kernel<T, EV>, kTileWarps * 32, plan->smem) !=
             cudaSuccess ||
         b < 1)
       b = 1;
@@ -1224,11 +1238,11 @@ static int tile_grid(TilePlan* plan, int* grid) {
   return 0;
 }
 
-template <typename T, int EV = PipeEV<T>::v, int G = 1>
+template <typename T, int EV = PipeEV<T>::v>
 static int launch_tile(const vbg_matrix* m, const ApplyArgs& a0, TilePlan* plan, cudaStream_t s) {
   constexpr bool f32 = std::is_same<T, float>::value;
   int grid = 0;
-  int rc = tile_grid<T, EV, G>(plan, &grid);
+  int rc = tile_grid<T, EV>(plan, &grid);
   if (rc) return rc;
   if ((rc = check_dot_ctas(a0, grid))) return rc;
   ApplyArgs a = a0;
@@ -1237,12 +1251,69 @@ static int launch_tile(const vbg_matrix* m, const ApplyArgs& a0, TilePlan* plan,
   a.span_koff32 = m->span_koff32.as<int64_t>();
   a.row_sptr = m->row_sptr.as<int>();
   const T* vals = (f32 ? m->valsK32 : m->valsK).as<T>();
-  apply_tile_kernel<T, EV, G><<<grid, kTileWarps * 32, plan->smem, s>>>(
+  apply_tile_kernel<T, EV><<<grid, kTileWarps * 32, plan->smem, s>>>(
       a, vals, plan->tiles.as<int4>(), plan->ranges.as<int4>(), plan->qidx.as<unsigned short>(),
       plan->rowinfo.as<int4>(), plan->ntiles, (unsigned)tile_vals_bytes(plan->vcap, (int)sizeof(T)),
       (unsigned)plan->qcap, tile_queue_on(m, a.ld, (int)sizeof(T)) ? plan->queue.as<int>() : nullptr, 0, grid);
   VBG_CUDA(cudaGetLastError());
   return 0;
+}
+
+template <int G>
+static int launch_narrow(const vbg_matrix* m, const ApplyArgs& a, TilePlan* plan, cudaStream_t s) {
+  static bool attr_set[kMaxDevices] = {};
+  const int dev = current_device();
+  if (!attr_set[dev]) {
+    VBG_CUDA(cudaFuncSetAttribute(apply_narrow_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)kTileSmemBudget32));
+    attr_set[dev] = true;
+  }
+  if (!plan->grid) {
+    int b = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, apply_narrow_kernel<G>, kTileWarps * 32, plan->smem) !=
+            cudaSuccess ||
+        b < 1)
+      b = 1;
+    plan->grid = std::max(1, std::min(plan->ntiles, b * sm_count()));
+  }
+  if (int rc = check_dot_ctas(a, plan->grid)) return rc;
+  apply_narrow_kernel<G><<<plan->grid, kTileWarps * 32, plan->smem, s>>>(
+      a, m->valsK32.as<float>(), plan->tiles.as<int4>(), plan->ranges.as<int4>(), plan->qidx.as<unsigned short>(),
+      plan->rowinfo.as<int4>(), plan->ntiles, (unsigned)tile_vals_bytes(plan->vcap, 4), (unsigned)plan->qcap,
+      (unsigned)narrow_stage_bytes(plan->vcap, plan->qcap, plan->xcap, a.ld * 4), 0, plan->grid);
+  VBG_CUDA(cudaGetLastError());
+  return 0;
+}
+
+template <typename T, int NP>
+static int launch_dtile_np(const vbg_matrix* m, const ApplyArgs& a, TilePlan* plan, cudaStream_t s) {
+  static bool attr_set[kMaxDevices] = {};
+  const int dev = current_device();
+  if (!attr_set[dev]) {
+    VBG_CUDA(cudaFuncSetAttribute(apply_dtile_kernel<T, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)kTileSmemBudget));
+    attr_set[dev] = true;
+  }
+  if (!plan->grid) {
+    int b = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, apply_dtile_kernel<T, NP>, kTileWarps * 32, plan->smem) !=
+            cudaSuccess ||
+        b < 1)
+      b = 1;
+    plan->grid = std::max(1, std::min(plan->ntiles, b * sm_count()));
+  }
+  if (int rc = check_dot_ctas(a, plan->grid)) return rc;
+  apply_dtile_kernel<T, NP><<<plan->grid, kTileWarps * 32, plan->smem, s>>>(
+      a, m->valsK.as<T>(), plan->tiles.as<int4>(), plan->xrows.as<int>(), plan->qidx.as<unsigned short>(),
+      plan->rowinfo.as<int4>(), plan->ntiles, (unsigned)tile_vals_bytes(plan->vcap, (int)sizeof(T)),
+      (unsigned)plan->qcap, 0, plan->grid);
+  VBG_CUDA(cudaGetLastError());
+  return 0;
+}
+
+template <typename T>
+static int launch_dtile(const vbg_matrix* m, const ApplyArgs& a, TilePlan* plan, cudaStream_t s) {
+  return dtile_pieces<T>(a.ld) == 1 ? launch_dtile_np<T, 1>(m, a, plan, s) : launch_dtile_np<T, 2>(m, a, plan, s);
 }
 
 // Whether this apply runs on apply_chain_kernel<T, EV, G>: the tiled
@@ -1305,14 +1376,10 @@ static int tile_prepare(const vbg_matrix* m, bool f32, int ld, cudaStream_t s) {
     if (ld != 16 && ld != 32 && ld != 64) return 0;
     rb = ld * 4;
     es = 4;
-  } else if (m->dtype == VBG_C128) {
-    if (ld != 32 * PipeEV<cplx>::v) return 0;
-    rb = 32 * 16;
-    es = 16;
   } else {
-    if (ld != 16 && ld != 32 * PipeEV<double>::v) return 0;
-    rb = ld * 8;
-    es = 8;
+    es = (int)elem_size(m->dtype);
+    if (ld * es != 128 && ld * es != 256 && ld * es != 512) return 0;
+    rb = ld * es;
   }
   if (chain_enabled(es)) {
     const int rc = chain_plan(m, rb, es, s, &cp);
@@ -1373,12 +1440,13 @@ static int launch_fwd_mv(const vbg_matrix* m, const ApplyArgs& a, const T* v, cu
     if (!any) return kNotApplicable;
   }
   if (any || which == VBG_KERNEL_TILE) {
-    if (tile_use<T>(m, false, a, s, allow_alloc, &tp)) return launch_tile<T>(m, a, tp, s);
     if constexpr (std::is_same<T, float>::value) {
-      if (tile_use<float, 1>(m, false, a, s, allow_alloc, &tp)) return launch_tile<float, 1>(m, a, tp, s);
-    }
-    if constexpr (!std::is_same<T, cplx>::value) {
-      if (tile_use<T, 1, 2>(m, false, a, s, allow_alloc, &tp)) return launch_tile<T, 1, 2>(m, a, tp, s);
+      if (tile_use<float>(m, false, a, s, allow_alloc, &tp)) return launch_tile<float>(m, a, tp, s);
+      if (tile_use<float, 4, 4>(m, false, a, s, allow_alloc, &tp)) return launch_narrow<4>(m, a, tp, s);
+      if (tile_use<float, 4, 8>(m, false, a, s, allow_alloc, &tp)) return launch_narrow<8>(m, a, tp, s);
+    } else {
+      if (tile_use<T>(m, false, a, s, allow_alloc, &tp))
+        return dtile_pieces<T>(a.ld) ? launch_dtile<T>(m, a, tp, s) : launch_tile<T>(m, a, tp, s);
     }
     if (!any) return kNotApplicable;
   }
@@ -1388,6 +1456,26 @@ static int launch_fwd_mv(const vbg_matrix* m, const ApplyArgs& a, const T* v, cu
   }
   if constexpr (std::is_same<T, float>::value) return launch_mv_t<float>(m, a, v, s);
   return launch_mma(m, false, a, s);
+}
+
+// The kernel of a forward multivector apply whose matrix has no tiles of at
+// least 8 block rows.  FP32: the pipelined kernel where it applies.  FP64 and
+// complex: tensor-core rows, whose cost goes with the number of m8n8k4 steps
+// (32 values each, however few a block fills), except on small blocks where
+// the pipelined kernel, whose cost goes with the values, fills whole warps
+// (rows of a multiple of 512 bytes), or whose real multiply-adds stand against
+// four steps a product (complex).  By the mean values of a block; us an apply,
+// pipelined / rows, 20000 block rows of 13 random blocks, real 64 columns:
+// sizes 2-4 (mean 9) 98 / 134, 3-5 (16) 109 / 152, 4-8 (36) 389 / 169; real
+// 128 columns 203 / 287, 229 / 311, 560 / 351; complex 16 columns 1-2 (2)
+// 77 / 106, 2-4 105 / 107, 3-5 121 / 117; real 32 columns 74 / 68, 89 / 70.
+template <typename T>
+static int untiled_choice(const vbg_matrix* m, const ApplyArgs& a, cudaStream_t s) {
+  constexpr bool f32 = std::is_same<T, float>::value, cx = std::is_same<T, cplx>::value;
+  const bool full = (int64_t)a.ld * (int)sizeof(T) % 512 == 0;
+  const double most = full ? 20.0 : cx ? 10.0 : 0.0;
+  const bool pipe = f32 || (double)m->nnz <= most * (double)m->nnzb;
+  return pipe && pipe_use<T>(m, false, a, s, true) ? VBG_KERNEL_PIPE : VBG_KERNEL_ROWS;
 }
 
 // The autotuner: the first forward multivector apply with a given leading
@@ -1421,9 +1509,21 @@ static int autotune_fwd(const vbg_matrix* m, const ApplyArgs& a0, const T* v, cu
   *choice = -1;
   auto* mm = const_cast<vbg_matrix*>(m);
   const auto cap_key = std::make_pair(a.ld, (int)sizeof(T));
-  for (int cand : {VBG_KERNEL_CHAIN, VBG_KERNEL_TILE, VBG_KERNEL_PIPE, VBG_KERNEL_ROWS}) {
-    // alone on this apply, or FP32: rows run only what no other kernel takes
-    if (cand == VBG_KERNEL_ROWS && (std::is_same<T, float>::value || *choice < 0)) break;
+  // Kernels that add a row's products in different orders are not timed
+  // against each other, so that equal matrices give equal bits whatever the
+  // clock said.  FP64 and complex values at 512-byte rows: tiles, chained or
+  // not (which add alike), where tiles of at least 8 block rows fit, else
+  // untiled_choice.  FP32 at 64 columns and up: as timed (the chained, tiled
+  // and pipelined forms add alike).
+  constexpr bool f32 = std::is_same<T, float>::value;
+  std::vector<int> cands = {VBG_KERNEL_CHAIN, VBG_KERNEL_TILE, VBG_KERNEL_PIPE};
+  TilePlan* tp = nullptr;
+  if constexpr (!f32) {
+    const bool tiles = tile_use<T>(m, false, a, s, true, &tp) && tp->rows >= 8;
+    if (tiles) cands = {VBG_KERNEL_CHAIN, VBG_KERNEL_TILE};
+    else cands.clear();
+  }
+  for (int cand : cands) {
     // the tiled kernel once per tile height cap (its own plan each) and per
     // tile order (fixed stride, work queue)
     for (int trial = 0; trial < 6; ++trial) {
@@ -1468,7 +1568,7 @@ static int autotune_fwd(const vbg_matrix* m, const ApplyArgs& a0, const T* v, cu
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  if (!rc && *choice < 0) *choice = VBG_KERNEL_ROWS;
+  if (!rc && *choice < 0) *choice = untiled_choice<T>(m, a, s);
   return rc;
 }
 
@@ -1490,8 +1590,26 @@ static int fwd_choice(const vbg_matrix* m, bool f32, const ApplyArgs& a, const T
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return 0;
   int choice = -1;
-  int rc = autotune_fwd<T>(m, a, v, s, &choice);
-  if (rc) return rc;
+  int rc = 0;
+  const bool narrow = std::is_same<T, float>::value && (a.ld == 16 || a.ld == 32);
+  if (dtile_pieces<T>(a.ld) != 0 || narrow) {
+    // by rule, not by trials (three plans cost more than they gain: within
+    // 5 % on lattices of 1.2k to 11k block rows): the tallest tiles that give
+    // every SM two, of at most 8 block rows on smaller matrices
+    const auto cap_key = std::make_pair(a.ld, (int)sizeof(T));
+    int cap = kTileRowsMax;
+    while (cap > 8 && m->n / cap < 2 * sm_count()) cap -= 4;
+    mm->tile_rows_cap[cap_key] = cap;
+    TilePlan* tp = nullptr;
+    bool tiles;
+    if constexpr (std::is_same<T, float>::value)
+      tiles = tile_use<float, 4, 4>(m, false, a, s, true, &tp) || tile_use<float, 4, 8>(m, false, a, s, true, &tp);
+    else
+      tiles = tile_use<T>(m, false, a, s, true, &tp);
+    choice = tiles && tp->rows >= 8 ? VBG_KERNEL_TILE : untiled_choice<T>(m, a, s);
+  } else if ((rc = autotune_fwd<T>(m, a, v, s, &choice))) {
+    return rc;
+  }
   mm->tuned[key] = choice;
   *which = choice;
   return 0;
@@ -2004,7 +2122,7 @@ int vbg_apply_kernel(const vbg_matrix* m, int ld, int precision, int* kernel) {
     chain = chain_ok && (chain_use<float>(m, a, nullptr, true, &cp) || chain_use<float, 1>(m, a, nullptr, true, &cp) ||
                          chain_use<float, 1, 2>(m, a, nullptr, true, &cp));
     tile = chain || tile_use<float>(m, false, a, nullptr, true, &tp) ||
-           tile_use<float, 1>(m, false, a, nullptr, true, &tp) || tile_use<float, 1, 2>(m, false, a, nullptr, true, &tp);
+           tile_use<float, 4, 4>(m, false, a, nullptr, true, &tp) || tile_use<float, 4, 8>(m, false, a, nullptr, true, &tp);
     pipe = tile || pipe_use<float>(m, false, a, nullptr, true);
   } else if (m->dtype == VBG_C128) {
     chain = chain_ok && chain_use<cplx>(m, a, nullptr, true, &cp);
@@ -2012,8 +2130,7 @@ int vbg_apply_kernel(const vbg_matrix* m, int ld, int precision, int* kernel) {
     pipe = tile || pipe_use<cplx>(m, false, a, nullptr, true);
   } else {
     chain = chain_ok && (chain_use<double>(m, a, nullptr, true, &cp) || chain_use<double, 1, 2>(m, a, nullptr, true, &cp));
-    tile = chain || tile_use<double>(m, false, a, nullptr, true, &tp) ||
-           tile_use<double, 1, 2>(m, false, a, nullptr, true, &tp);
+    tile = chain || tile_use<double>(m, false, a, nullptr, true, &tp);
     pipe = tile || pipe_use<double>(m, false, a, nullptr, true);
   }
   *kernel = chain ? VBG_KERNEL_CHAIN : tile ? VBG_KERNEL_TILE : pipe ? VBG_KERNEL_PIPE : VBG_KERNEL_ROWS;
@@ -2255,7 +2372,8 @@ int vbg_kpm_moments(const vbg_matrix* m, int R, int ld, const void* V0, int M, i
   if (R > 1 && m->max_bs <= kPipeMaxBs && (f32 ? pipe_groups<float>(ldw) : pipe_groups<double>(ldw)) != 0) {
     if ((rc = ensure_kernel_layout(m, f32, s))) return rc;
     if ((rc = ensure_spans(m, pipe_span_cap(m), s))) return rc;
-    if ((rc = tile_prepare(m, f32, ldw, s))) return rc;
+    // (with the autotuner on, tune_recurrence makes the plan it wants)
+    if (!(g_opt_autotune.load() && g_opt_chain.load() == 2) && (rc = tile_prepare(m, f32, ldw, s))) return rc;
   }
   // the kernel choice, before a graph capture freezes it
   if (f32)
@@ -2453,7 +2571,8 @@ int vbg_kpm_moments_batched(const vbg_matrix* m, int nseg, const int* seg_rows, 
   if (m->max_bs <= kPipeMaxBs && (f32 ? pipe_groups<float>(ldw) : pipe_groups<double>(ldw)) != 0) {
     if ((rc = ensure_kernel_layout(m, f32, s))) return rc;
     if ((rc = ensure_spans(m, pipe_span_cap(m), s))) return rc;
-    if ((rc = tile_prepare(m, f32, ldw, s))) return rc;
+    // (with the autotuner on, tune_recurrence makes the plan it wants)
+    if (!(g_opt_autotune.load() && g_opt_chain.load() == 2) && (rc = tile_prepare(m, f32, ldw, s))) return rc;
   }
   if ((rc = ensure_grid_scratch(m))) return rc;
   if (f32)

@@ -177,10 +177,12 @@ struct TilePlan {
   int grid = 0, smem = 0;
   // four int4 per tile: {first block row, end block row, first range, end
   // range}, {first value offset (two halves), value bytes, X bytes}, {shared
-  // row of the first own X row, own scalar rows, first own scalar row, 0},
+  // row of the first own X row, own scalar rows, first own scalar row, first
+  // entry of xrows},
   // {first q-list entry staged, q-list bytes, 0, 0}
   DevBuf tiles;
   DevBuf ranges;      // int4 {first X row, X rows, first shared-memory row, 0}
+  DevBuf xrows;       // tensor-core form: the tile's X rows in shared-memory order
   // The q-list: per block row, the shared-memory row of every X row its
   // blocks read, in slot order and column order within a block (uint16;
   // each row's list starts at a multiple of 4 entries).

@@ -1,9 +1,9 @@
 // Row-wise multivector apply on the FP64 tensor cores: Y = A X and Y = A^H X
 // with the fused epilogue, real and complex, any block sizes and any leading
 // dimension.  It runs what the staged applies (vbg_pipe.cuh, vbg_tile.cuh,
-// vbg_chain.cuh) do not take -- the adjoint, blocks over 8, leading
-// dimensions that are no lane-group width -- and is one of the autotuner's
-// candidates for the rest.
+// vbg_dtile.cuh, vbg_chain.cuh) do not take -- the adjoint, blocks over 8,
+// leading dimensions that are no lane-group width -- and matrices without
+// tiles unless their blocks are small (untiled_choice).
 //
 // A warp multiplies one task: 8 MT scalar rows of one block row against NP
 // column pieces of 128 bytes (16 real or 8 complex columns), by m8n8k4

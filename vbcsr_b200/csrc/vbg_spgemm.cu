@@ -17,11 +17,12 @@
 // global-memory table for rows too wide for it), so every column's sum is
 // formed in the reference's order with separately rounded products and adds
 // -- the kept pattern is the reference's bit for bit.  Kept columns are
-// compacted with warp ballots and bitonic-sorted.  Numeric: the warp maps
-// C's columns in a table, then each lane multiplies one (A_ik, B_kj) block
-// pair into its destination block; the Frobenius norms of the finished row
-// are computed in the same kernel (the filter's keep flags), and the kept
-// blocks are compacted afterwards.
+// compacted with warp ballots and bitonic-sorted.  Numeric: FP64 and complex
+// blocks of at most 8 x 8 on the tensor cores (vbg_numeric.cu); FP32 values and
+// larger blocks here, a warp per work item of up to kNumItem blocks of one C
+// row.  The Frobenius norms of the finished blocks are computed in the same
+// kernel (the filter's keep flags), and the kept blocks are compacted
+// afterwards.
 #include <algorithm>
 #include <cstring>
 #include <numeric>
@@ -412,8 +413,7 @@ struct BlockAcc {
 // One C block C_ij (slot p; its row has r scalar rows) of the numeric phase: the
 // kept pairs of A's row and B's column j, multiplied and written, the keep
 // flag (and with GATED the pair-norm bound) stored.  span > 0: A's row is
-// mapped in wtab (column kmin + d -> slot).  A's value at offset o is A[o]
-// (the row kernel passes a base that puts A's row in shared memory).
+// mapped in wtab (column kmin + d -> slot).  A's value at offset o is A[o].
 template <typename T, int R, bool GATED>
 __device__ __forceinline__ void numeric_block(const NumArgs& a, const T* __restrict__ A, const T* __restrict__ B,
                                               T* __restrict__ C, int p, int r, int a0, int a1, int kmin, int span,

@@ -4,9 +4,11 @@
 //
 // Y = A X (+ the fused epilogue of vbg_cheb_step) for multivectors whose
 // padded row is exactly one warp of 16-byte (FP64, complex) or 8-byte (FP32)
-// pieces -- k = 64 FP64 / FP32, k = 32 complex -- and blocks of at most
-// 8 x 8, when the matrix's rows can be cut into tiles whose working set fits
-// shared memory.
+// pieces -- k = 64 FP64 / FP32, k = 32 complex -- or 16 or 32 FP32 columns
+// (apply_narrow_kernel at the end), and blocks of at most 8 x 8, when the
+// matrix's rows can be cut into tiles whose working set fits shared memory.
+// FP64 and complex rows of 128 and 256 bytes take the same tiles through the
+// tensor cores (vbg_dtile.cuh).
 //
 // A tile is up to kTileRowsMax consecutive block rows.  The block columns its
 // blocks touch form a few contiguous ranges for matrices whose neighbours
@@ -23,9 +25,9 @@
 // column order, that row's place in the staged X (16-bit, read four at a
 // time).  A warp walks it with one shared-memory load of the lane's piece of
 // X, the column's values (a broadcast) and R x EV multiply-adds per X row:
-// no per-block records, shuffles or switches.  For multivectors of half a
-// warp's width (16 FP64 or FP32 columns) two lane groups each take every
-// other X row and add their sums by a shuffle.
+// no per-block records, shuffles or switches.  In the chained form, for
+// multivectors of half a warp's width (16 FP64 or FP32 columns), two lane
+// groups each take every other X row and add their sums by a shuffle.
 //
 // The host plans the tiles once per structure (tile_plan): the tallest
 // height in {16, 12, 10, 8, 6, 4} whose largest tile fits the budget, each
@@ -52,6 +54,19 @@ __host__ __device__ inline size_t tile_vals_bytes(int64_t vcap, int ves) {
 }
 __host__ __device__ inline size_t tile_smem_bytes(int64_t vcap, int ves, int qcap, int xcap, int rb) {
   return 16 + tile_vals_bytes(vcap, ves) + (size_t)qcap + (size_t)xcap * rb;
+}
+
+// Narrow FP32 rows (16 and 32 columns) run on apply_narrow_kernel, which stages
+// the next tile while it multiplies one: two stages of {tile record, row
+// records, values, q-list, X rows}.
+__host__ __device__ inline bool tile_narrow(int rb, int ves) { return ves == 4 && rb <= 128; }
+constexpr int kNarrowHead = 64 + kTileRowsMax * 16;  // records of a stage
+__host__ __device__ inline size_t narrow_stage_bytes(int64_t vcap, int qcap, int xcap, int rb) {
+  return (size_t)kNarrowHead + tile_vals_bytes(vcap, 4) + (size_t)qcap + (size_t)xcap * rb;
+}
+__host__ __device__ inline size_t tile_plan_smem(int64_t vcap, int ves, int qcap, int xcap, int rb) {
+  return tile_narrow(rb, ves) ? 16 + 2 * narrow_stage_bytes(vcap, qcap, xcap, rb)
+                              : tile_smem_bytes(vcap, ves, qcap, xcap, rb);
 }
 
 // Splits the block rows [0, T) of a tile (work w[i] each) into at most W
@@ -185,7 +200,7 @@ static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, Tile
       qcap = std::max(qcap, qlist_bytes(qstart, t0, t1));
       // shared-memory rows are 16-bit q-list entries
       fits = (int)ranges.size() <= kTileMaxRanges && xcap <= 65535 &&
-             tile_smem_bytes(vcap, ves, qcap, (int)xcap, rb) <= (ves == 4 ? kTileSmemBudget32 : kTileSmemBudget);
+             tile_plan_smem(vcap, ves, qcap, (int)xcap, rb) <= (ves == 4 ? kTileSmemBudget32 : kTileSmemBudget);
     }
     if (fits) {
       plan->rows = tr;
@@ -203,6 +218,8 @@ static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, Tile
   const int tr = plan->rows;
   const int ntiles = (n + tr - 1) / tr;
   std::vector<int4> h_tiles(4 * (size_t)ntiles), h_ranges, h_rowinfo(std::max(n, 1));
+  const bool steps = ves > 4 && rb <= 256;  // runs on the tensor-core form (vbg_dtile.cuh)
+  std::vector<int> h_xrows;  // of which: the staged X rows one by one
   // the q-list, padded so that the last tile's staged slice stays inside
   std::vector<unsigned short> h_qidx(((size_t)qstart[n] + 7) / 8 * 8 + 8, 0);
   int64_t k0 = 0;  // kernel-layout value offset of the tile's first slot
@@ -217,6 +234,10 @@ static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, Tile
       dst += cnt;
     }
     const int rend = (int)h_ranges.size();
+    const int xoff = (int)h_xrows.size();
+    if (steps)
+      for (int k = rbeg; k < rend; ++k)
+        for (int x = 0; x < h_ranges[k].y; ++x) h_xrows.push_back(h_ranges[k].x + x);
     // the shared-memory row of a staged X row
     auto srow_of = [&](int x) {
       int lo = rbeg, hi = rend - 1;
@@ -237,14 +258,16 @@ static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, Tile
         const int x0 = (int)soff[ci[p]];
         for (int q = 0; q < bsz[ci[p]]; ++q) h_qidx[k++] = (unsigned short)srow_of(x0 + q);
       }
-      h_rowinfo[i] = make_int4(qstart[i] - qb, qn[i], (int)vs, bsz[i]);
+      // narrow: the row's first scalar row within the tile beside its size
+      h_rowinfo[i] = make_int4(qstart[i] - qb, qn[i], (int)vs,
+                               bsz[i] | (tile_narrow(rb, ves) ? (int)(soff[i] - soff[t0]) << 8 : 0));
       vs += vrow[i];
     }
     // the tile's rows in runs of consecutive rows, one run per warp, with
     // balanced work (the multiply-adds and loads of a row: its X rows times
-    // its size plus a few)
+    // its size plus a few; in tensor-core steps of four X rows and an epilogue)
     int64_t wk[kTileRowsMax];
-    for (int i = t0; i < t1; ++i) wk[i - t0] = (int64_t)qn[i] * (bsz[i] + 2) + 8;
+    for (int i = t0; i < t1; ++i) wk[i - t0] = steps ? (qn[i] + 3) / 4 + 6 : (int64_t)qn[i] * (bsz[i] + 2) + 8;
     int bounds[kTileWarps];
     balanced_runs(wk, t1 - t0, kTileWarps, bounds);
     unsigned packed[2] = {0u, 0u};
@@ -252,20 +275,23 @@ static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, Tile
     const int ys0 = (int)soff[t0], own = (int)(soff[t1] - soff[t0]);
     h_tiles[4 * (size_t)t] = make_int4(t0, t1, rbeg, rend);
     h_tiles[4 * (size_t)t + 1] = make_int4((int)(k0 & 0xffffffff), (int)(k0 >> 32), (int)(vs * ves), dst * rb);
-    h_tiles[4 * (size_t)t + 2] = make_int4(srow_of(ys0), own, ys0, 0);
+    h_tiles[4 * (size_t)t + 2] = make_int4(srow_of(ys0), own, ys0, xoff);
     h_tiles[4 * (size_t)t + 3] = make_int4(qb, qlist_bytes(qstart, t0, t1), (int)packed[0], (int)packed[1]);
     k0 += vs;
   }
   plan->ntiles = ntiles;
-  plan->smem = (int)tile_smem_bytes(plan->vcap, ves, plan->qcap, plan->xcap, rb);
+  plan->smem = (int)tile_plan_smem(plan->vcap, ves, plan->qcap, plan->xcap, rb);
   if ((rc = plan->tiles.ensure(h_tiles.size() * sizeof(int4), s))) return rc;
   if ((rc = plan->ranges.ensure(std::max<size_t>(h_ranges.size(), 1) * sizeof(int4), s))) return rc;
+  if ((rc = plan->xrows.ensure(std::max<size_t>(h_xrows.size(), 1) * sizeof(int), s))) return rc;
   if ((rc = plan->qidx.ensure(h_qidx.size() * sizeof(unsigned short), s))) return rc;
   if ((rc = plan->rowinfo.ensure(h_rowinfo.size() * sizeof(int4), s))) return rc;
   VBG_CUDA(cudaMemcpyAsync(plan->tiles.p, h_tiles.data(), h_tiles.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
   if (!h_ranges.empty())
     VBG_CUDA(cudaMemcpyAsync(plan->ranges.p, h_ranges.data(), h_ranges.size() * sizeof(int4), cudaMemcpyHostToDevice,
                              s));
+  if (!h_xrows.empty())
+    VBG_CUDA(cudaMemcpyAsync(plan->xrows.p, h_xrows.data(), h_xrows.size() * sizeof(int), cudaMemcpyHostToDevice, s));
   VBG_CUDA(cudaMemcpyAsync(plan->qidx.p, h_qidx.data(), h_qidx.size() * sizeof(unsigned short),
                            cudaMemcpyHostToDevice, s));
   VBG_CUDA(cudaMemcpyAsync(plan->rowinfo.p, h_rowinfo.data(), h_rowinfo.size() * sizeof(int4), cudaMemcpyHostToDevice,
@@ -418,6 +444,120 @@ __device__ __forceinline__ void qlist_row_r(int r, const unsigned short* ql, int
   }
 }
 
+// Narrow FP32 multivectors (16 or 32 columns): four columns per lane, so a row
+// of X is 32 / G = 4 or 8 lanes wide and the G = 8 or 4 lane groups take G
+// X rows of the q-list at once.  A step loads the lane's 16 bytes of X and its
+// X row's values (one address per group: a 128-byte pass) for 4 R
+// multiply-adds; with one column per lane and two groups the same loads fed
+// R (41 instructions per two X rows, 60 % issue: instruction-bound).
+// nq q-list entries; acc[o] this lane's four columns of row o, not yet summed
+// over the groups.
+template <int R, int G>
+__device__ __forceinline__ void narrow_row(const unsigned short* ql, int nq, const float* vr, const unsigned char* xl,
+                                           int grp, float (&acc)[kPipeMaxBs][4]) {
+  constexpr int RB = 32 / G * 16;
+  constexpr int RP = kernel_layout_rows(R, 4);
+#pragma unroll
+  for (int o = 0; o < R; ++o)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) acc[o][u] = 0.0f;
+  auto step = [&](int q) {
+    const float4 x = *reinterpret_cast<const float4*>(xl + (unsigned)ql[q] * RB);
+    const float4* w = reinterpret_cast<const float4*>(vr + q * RP);
+#pragma unroll
+    for (int j = 0; j < RP / 4; ++j) {
+      const float4 v = w[j];
+      const float vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+        if (4 * j + t < R) {
+          acc[4 * j + t][0] = fmaf(vv[t], x.x, acc[4 * j + t][0]);
+          acc[4 * j + t][1] = fmaf(vv[t], x.y, acc[4 * j + t][1]);
+          acc[4 * j + t][2] = fmaf(vv[t], x.z, acc[4 * j + t][2]);
+          acc[4 * j + t][3] = fmaf(vv[t], x.w, acc[4 * j + t][3]);
+        }
+    }
+  };
+  int b = 0;
+#pragma unroll 2
+  for (; b + G <= nq; b += G) step(b + grp);
+  if (b + grp < nq) step(b + grp);
+}
+
+// Sums acc over the lane groups: lane bits 4 and 3 choose which of the lane's
+// four columns it keeps (so each exchange halves what is left), and for 16
+// columns bit 2 which of two neighbouring rows.  out[i]: the lane's column
+// 4 gl + 2 bit4 + bit3 of row i (32 columns) or of row 2 i + bit2 (16).
+template <int R, int G>
+__device__ __forceinline__ void narrow_sum(const float (&acc)[kPipeMaxBs][4], int lane, float (&out)[kPipeMaxBs]) {
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+  auto fold = [&](float lo, float hi, bool up, int off) {  // keep hi if up, add the partner's
+    const float send = up ? lo : hi, mine = up ? hi : lo;
+    return mine + __shfl_xor_sync(0xffffffffu, send, off);
+  };
+  float c[kPipeMaxBs];
+#pragma unroll
+  for (int o = 0; o < R; ++o) {
+    const float e = fold(acc[o][0], acc[o][2], b4, 16), f = fold(acc[o][1], acc[o][3], b4, 16);
+    c[o] = fold(e, f, b3, 8);
+  }
+  if constexpr (G == 8) {
+#pragma unroll
+    for (int i = 0; i < (R + 1) / 2; ++i) out[i] = fold(c[2 * i], 2 * i + 1 < R ? c[2 * i + 1] : 0.0f, b2, 4);
+  } else {
+#pragma unroll
+    for (int o = 0; o < R; ++o) out[o] = c[o];
+  }
+}
+
+// One block row of a narrow FP32 tile with its epilogue (tile_epilogue's, one
+// element per lane and output row).
+template <int R, int G>
+__device__ __forceinline__ void narrow_block_row(const ApplyArgs& a, const unsigned short* ql, int nq, const float* vr,
+                                                 const unsigned char* xs, int oslot, long long y0, int lane, double& d0,
+                                                 double& d1) {
+  constexpr int LG = 32 / G;  // lanes per X row
+  constexpr int LD = LG * 4;
+  const int gl = lane % LG, grp = lane / LG;
+  float acc[kPipeMaxBs][4], out[kPipeMaxBs];
+  narrow_row<R, G>(ql, nq, vr, xs + gl * 16, grp, acc);
+  narrow_sum<R, G>(acc, lane, out);
+  const int col = 4 * gl + ((lane & 16) ? 2 : 0) + ((lane & 8) ? 1 : 0);
+  constexpr int STEP = G == 8 ? 2 : 1;
+#pragma unroll
+  for (int i = 0; i < (R + STEP - 1) / STEP; ++i) {
+    const int o = STEP * i + (G == 8 && (lane & 4) ? 1 : 0);
+    if (o >= R) continue;
+    const long long el = (y0 + o) * LD + col;
+    const float x = *reinterpret_cast<const float*>(xs + (size_t)(oslot + o) * (LG * 16) + col * 4);
+    float y = scal_r(a.alpha, out[i]);
+    if (a.beta != 0.0) y = axpy_r(a.beta, x, y);
+    if (a.gamma != 0.0) y = axpy_r(a.gamma, static_cast<const float*>(a.Xprev)[el], y);
+    if (a.want_dots) {
+      d0 += re_dot(a.dotw ? static_cast<const float*>(a.dotw)[el] : x, y);
+      d1 += re_dot(y, y);
+    }
+    if (a.acc) static_cast<float*>(a.acc)[el] = cmad(a.cre, a.cim, y, static_cast<const float*>(a.acc)[el]);
+    static_cast<float*>(a.Y)[el] = y;
+  }
+}
+
+template <int G>
+__device__ __forceinline__ void narrow_block_row_r(int r, const ApplyArgs& a, const unsigned short* ql, int nq,
+                                                   const float* vr, const unsigned char* xs, int oslot, long long y0,
+                                                   int lane, double& d0, double& d1) {
+  switch (r) {
+    case 1: narrow_block_row<1, G>(a, ql, nq, vr, xs, oslot, y0, lane, d0, d1); break;
+    case 2: narrow_block_row<2, G>(a, ql, nq, vr, xs, oslot, y0, lane, d0, d1); break;
+    case 3: narrow_block_row<3, G>(a, ql, nq, vr, xs, oslot, y0, lane, d0, d1); break;
+    case 4: narrow_block_row<4, G>(a, ql, nq, vr, xs, oslot, y0, lane, d0, d1); break;
+    case 5: narrow_block_row<5, G>(a, ql, nq, vr, xs, oslot, y0, lane, d0, d1); break;
+    case 6: narrow_block_row<6, G>(a, ql, nq, vr, xs, oslot, y0, lane, d0, d1); break;
+    case 7: narrow_block_row<7, G>(a, ql, nq, vr, xs, oslot, y0, lane, d0, d1); break;
+    default: narrow_block_row<8, G>(a, ql, nq, vr, xs, oslot, y0, lane, d0, d1); break;
+  }
+}
+
 // Resident CTAs per SM the register allocation is held to: FP32 tiles need
 // half the shared memory of FP64 ones, so a third CTA fits when the kernel
 // keeps to 80 registers (measured: 503k against 396k moment-vectors/s on the
@@ -431,17 +571,16 @@ template <> struct TileMinCtas<float> { static constexpr int v = 3; };
 // barrier | values (vbytes16) | q-list (qbytes16) | X rows.  The next tile's
 // record is loaded while this one is multiplied; a warp's first row record
 // while the tile's copies are in flight.
-template <typename T, int EV, int G = 1>
+template <typename T, int EV>
 __global__ void __launch_bounds__(kTileWarps * 32, TileMinCtas<T>::v)
     apply_tile_kernel(ApplyArgs a, const T* __restrict__ vals, const int4* __restrict__ tiles,
                       const int4* __restrict__ ranges, const unsigned short* __restrict__ qidx,
                       const int4* __restrict__ rowinfo, int ntiles, unsigned vbytes16, unsigned qbytes16,
                       int* __restrict__ queue, int part_base, int total) {
   using L = PipeLane<T, EV>;
-  constexpr int RB = 32 / G * (int)sizeof(L);  // bytes of one X row (32 / G lanes)
+  constexpr int RB = 32 * (int)sizeof(L);  // bytes of one X row
   extern __shared__ __align__(16) unsigned char tile_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int gl = lane % (32 / G), grp = lane / (32 / G);  // lane within its group, the group
   const unsigned bar = smem_addr(tile_smem);
   const T* vs_base = reinterpret_cast<const T*>(tile_smem + 16);
   const unsigned short* qs_base = reinterpret_cast<const unsigned short*>(tile_smem + 16 + vbytes16);
@@ -531,12 +670,12 @@ __global__ void __launch_bounds__(kTileWarps * 32, TileMinCtas<T>::v)
         y0 = a.scal_off[row];
       }
       const int r = ri.w;
-      L acc[kPipeMaxBs];
-      qlist_row_r<T, EV, G>(r, qs_base + ri.x, ri.y, vs_base + ri.z, xs_base + (size_t)gl * sizeof(L), acc, grp);
       const int orow = (int)(y0 - tc.z);  // this row's first scalar row within the tile
       double rd0 = 0.0, rd1 = 0.0;
-      tile_epilogue<T, EV, RB, G>(a, acc, r, y0, gl, xs_base + (size_t)(tc.x + orow) * RB + (size_t)gl * sizeof(L),
-                                  rd0, rd1, grp);
+      L acc[kPipeMaxBs];
+      qlist_row_r<T, EV>(r, qs_base + ri.x, ri.y, vs_base + ri.z, xs_base + (size_t)lane * sizeof(L), acc, 0);
+      tile_epilogue<T, EV, RB>(a, acc, r, y0, lane, xs_base + (size_t)(tc.x + orow) * RB + (size_t)lane * sizeof(L),
+                               rd0, rd1, 0);
       if (a.want_dots) {
         if (a.row_dots) {
           write_row_dots(a.row_dots, row, rd0, rd1);
@@ -564,6 +703,118 @@ __global__ void __launch_bounds__(kTileWarps * 32, TileMinCtas<T>::v)
       queue[1] = 0;
       __threadfence();
     }
+  }
+  if (a.want_dots && !a.row_dots) grid_reduce2(d0, d1, a.partials, a.counter, a.dots_out, part_base, total);
+}
+
+// The tiled apply of narrow FP32 multivectors: persistent CTAs over the tiles in
+// a fixed stride, two stages.  Warp 0 issues the next tile's copies (a lane
+// per range of X) before it multiplies its share of this one, so that the
+// copies' latency is behind a tile's work; with one stage the warps waited
+// for it at every tile (4 of 9 cycles between issues at the barrier).  The
+// tile's and the rows' records come with the copies.
+template <int G>
+__global__ void __launch_bounds__(kTileWarps * 32, 3)
+    apply_narrow_kernel(ApplyArgs a, const float* __restrict__ vals, const int4* __restrict__ tiles,
+                        const int4* __restrict__ ranges, const unsigned short* __restrict__ qidx,
+                        const int4* __restrict__ rowinfo, int ntiles, unsigned vbytes16, unsigned qbytes16,
+                        unsigned stage_bytes, int part_base, int total) {
+  constexpr int RB = 32 / G * 16;
+  extern __shared__ __align__(16) unsigned char tile_smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned bar0 = smem_addr(tile_smem);
+  if (threadIdx.x == 0) {
+    mbar_init(bar0, 1);
+    mbar_init(bar0 + 8, 1);
+    mbar_init_fence();
+  }
+  __syncthreads();
+  const float* X = static_cast<const float*>(a.X);
+  const bool use_p = a.gamma != 0.0, use_d = a.want_dots && a.dotw;
+  int4 ra, rb, rc, rq;  // warp 0: the record of the next tile to issue
+  auto fetch = [&](int t) {
+    ra = tiles[4 * (size_t)t];
+    rb = tiles[4 * (size_t)t + 1];
+    rc = tiles[4 * (size_t)t + 2];
+    rq = tiles[4 * (size_t)t + 3];
+  };
+  auto issue = [&](int t, int k) {  // warp 0: tile t (record fetched) into stage k & 1
+    const unsigned st = bar0 + 16 + (unsigned)(k & 1) * stage_bytes, bar = bar0 + 8 * (k & 1);
+    // the stage's earlier shared-memory reads come before these copies
+    fence_proxy_async();
+    if (lane == 0) {
+      const unsigned rbytes = (unsigned)(ra.y - ra.x) * 16, vbytes = (unsigned)rb.z, obytes = (unsigned)rc.y * RB;
+      const long long k0 = (static_cast<long long>(rb.y) << 32) | static_cast<unsigned>(rb.x);
+      mbar_arm(bar, 64 + rbytes + vbytes + (unsigned)rq.y + (unsigned)rb.w);
+      bulk_g2s(st, tiles + 4 * (size_t)t, 64, bar);
+      bulk_g2s(st + 64, rowinfo + ra.x, rbytes, bar);
+      if (vbytes) bulk_g2s(st + kNarrowHead, vals + k0, vbytes, bar);
+      if (rq.y) bulk_g2s(st + kNarrowHead + vbytes16, qidx + rq.x, (unsigned)rq.y, bar);
+      // the epilogue's streamed operands: have L2 fetch the tile's rows
+      if (use_p) bulk_prefetch_l2(static_cast<const float*>(a.Xprev) + (long long)rc.z * a.ld, obytes);
+      if (use_d) bulk_prefetch_l2(static_cast<const float*>(a.dotw) + (long long)rc.z * a.ld, obytes);
+    }
+    __syncwarp();  // armed before any copy can complete
+    for (int g = ra.z + lane; g < ra.w; g += 32) {
+      const int4 rg = ranges[g];
+      bulk_g2s(st + kNarrowHead + vbytes16 + qbytes16 + (unsigned)rg.z * RB, X + (long long)rg.x * a.ld,
+               (unsigned)rg.y * RB, bar);
+    }
+  };
+  double d0 = 0.0, d1 = 0.0;
+  const int stride = gridDim.x;
+  int tile = blockIdx.x;
+  if (warp == 0 && tile < ntiles) {
+    fetch(tile);
+    issue(tile, 0);
+    if (tile + stride < ntiles) fetch(tile + stride);
+  }
+  bool failed = false;
+  for (int k = 0; tile < ntiles; ++k, tile += stride) {
+    if (warp == 0 && tile + stride < ntiles) {
+      issue(tile + stride, k + 1);
+      if (tile + 2 * stride < ntiles) fetch(tile + 2 * stride);
+    }
+    const unsigned bar = bar0 + 8 * (k & 1), parity = (unsigned)(k >> 1) & 1u;
+    const bool ok = warp == 0 ? pipe_wait(bar, parity) : true;
+    if (!__syncthreads_and(ok)) {
+      failed = true;
+      break;
+    }
+    (void)mbar_try_wait(bar, parity);
+    const unsigned char* st = tile_smem + 16 + (size_t)(k & 1) * stage_bytes;
+    const int4* rec = reinterpret_cast<const int4*>(st);
+    const int4* rows = reinterpret_cast<const int4*>(st + 64);
+    const float* vs = reinterpret_cast<const float*>(st + kNarrowHead);
+    const unsigned short* qs = reinterpret_cast<const unsigned short*>(st + kNarrowHead + vbytes16);
+    const unsigned char* xs = st + kNarrowHead + vbytes16 + qbytes16;
+    const int row0 = rec[0].x, ys0 = rec[2].z, own = rec[2].x;
+    const unsigned char* ends = reinterpret_cast<const unsigned char*>(rec + 3) + 8;  // of the warps' runs
+    const int i1 = ends[warp];
+    for (int i = warp == 0 ? 0 : ends[warp - 1]; i < i1; ++i) {
+      const int4 ri = rows[i];
+      const int r = ri.w & 0xff, orow = ri.w >> 8;
+      double rd0 = 0.0, rd1 = 0.0;
+      narrow_block_row_r<G>(r, a, qs + ri.x, ri.y, vs + ri.z, xs, own + orow, (long long)ys0 + orow, lane, rd0, rd1);
+      if (a.want_dots) {
+        if (a.row_dots) {
+          write_row_dots(a.row_dots, row0 + i, rd0, rd1);
+        } else {
+          d0 += rd0;
+          d1 += rd1;
+        }
+      }
+    }
+    __syncthreads();  // every warp is done with the stage before it is filled again
+  }
+  if (failed && warp == 0) {
+    if (lane == 0) atomicOr(&g_pipe_status, 1u);
+    // copies may still be in flight: both stages' (a stage that was never
+    // armed again has completed its phase)
+    mbar_wait_bounded(bar0, 0u);
+    mbar_wait_bounded(bar0, 1u);
+    mbar_wait_bounded(bar0 + 8, 0u);
+    mbar_wait_bounded(bar0 + 8, 1u);
   }
   if (a.want_dots && !a.row_dots) grid_reduce2(d0, d1, a.partials, a.counter, a.dots_out, part_base, total);
 }
