@@ -111,3 +111,25 @@ def test_fp32_tiles(oracle, dev, n, k):
     assert np.abs(mu - ref).max() / abs(ref[0]) < 2e-6
     assert np.array_equal(mu, _gpu.kpm_moments(_gpu.dmat(H), V, 8, precision=1))
     assert _capi.device_status(clear=True) == 0
+
+
+@pytest.mark.parametrize("n,lo,hi", [(37, 8, 8), (1500, 1, 2), (1501, 4, 8), (5003, 3, 5)])
+@pytest.mark.parametrize("k", [16, 32])
+def test_fp32_short_tiles(oracle, dev, n, lo, hi, k):
+    """Random patterns, whose tiles are too short for two stages (but for the
+    smallest matrix); tolerance as above, rows of 13 blocks of at most 8."""
+    from vbcsr_b200 import _capi
+
+    from . import _gpu
+
+    H = W.random_pattern(n, lo, hi, 12, seed=n)
+    H.values = (H.values - 0.5) / W.gershgorin_bound(H)
+    V = np.where(np.random.default_rng(k).random((H.N, k)) < 0.5, -1.0, 1.0)
+    dm = _gpu.dmat(H)
+    mu = _gpu.kpm_moments(dm, V, 8, precision=1)
+    assert _capi.apply_kernel(dm, k, precision=1) == "tile"
+    assert n == 37 or _capi.apply_tile_rows(dm, k, precision=1) < 8
+    ref = oracle.kpm_moments(H, V, 8, True)
+    assert np.abs(mu - ref).max() / abs(ref[0]) < 2e-6
+    assert np.array_equal(mu, _gpu.kpm_moments(_gpu.dmat(H), V, 8, precision=1))
+    assert _capi.device_status(clear=True) == 0

@@ -1259,30 +1259,35 @@ static int launch_tile(const vbg_matrix* m, const ApplyArgs& a0, TilePlan* plan,
   return 0;
 }
 
-template <int G>
-static int launch_narrow(const vbg_matrix* m, const ApplyArgs& a, TilePlan* plan, cudaStream_t s) {
+template <int G, int S>
+static int launch_narrow_s(const vbg_matrix* m, const ApplyArgs& a, TilePlan* plan, cudaStream_t s) {
   static bool attr_set[kMaxDevices] = {};
   const int dev = current_device();
   if (!attr_set[dev]) {
-    VBG_CUDA(cudaFuncSetAttribute(apply_narrow_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    VBG_CUDA(cudaFuncSetAttribute(apply_narrow_kernel<G, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)kTileSmemBudget32));
     attr_set[dev] = true;
   }
   if (!plan->grid) {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, apply_narrow_kernel<G>, kTileWarps * 32, plan->smem) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, apply_narrow_kernel<G, S>, kTileWarps * 32, plan->smem) !=
             cudaSuccess ||
         b < 1)
       b = 1;
     plan->grid = std::max(1, std::min(plan->ntiles, b * sm_count()));
   }
   if (int rc = check_dot_ctas(a, plan->grid)) return rc;
-  apply_narrow_kernel<G><<<plan->grid, kTileWarps * 32, plan->smem, s>>>(
+  apply_narrow_kernel<G, S><<<plan->grid, kTileWarps * 32, plan->smem, s>>>(
       a, m->valsK32.as<float>(), plan->tiles.as<int4>(), plan->ranges.as<int4>(), plan->qidx.as<unsigned short>(),
       plan->rowinfo.as<int4>(), plan->ntiles, (unsigned)tile_vals_bytes(plan->vcap, 4), (unsigned)plan->qcap,
       (unsigned)narrow_stage_bytes(plan->vcap, plan->qcap, plan->xcap, a.ld * 4), 0, plan->grid);
   VBG_CUDA(cudaGetLastError());
   return 0;
+}
+
+template <int G>
+static int launch_narrow(const vbg_matrix* m, const ApplyArgs& a, TilePlan* plan, cudaStream_t s) {
+  return plan->stages == 2 ? launch_narrow_s<G, 2>(m, a, plan, s) : launch_narrow_s<G, 1>(m, a, plan, s);
 }
 
 template <typename T, int NP>
@@ -1458,8 +1463,9 @@ static int launch_fwd_mv(const vbg_matrix* m, const ApplyArgs& a, const T* v, cu
   return launch_mma(m, false, a, s);
 }
 
-// The kernel of a forward multivector apply whose matrix has no tiles of at
-// least 8 block rows.  FP32: the pipelined kernel where it applies.  FP64 and
+// The kernel of a forward multivector apply whose matrix has no tiles (FP64 and
+// complex: none of at least 8 block rows).  FP32: the pipelined kernel where it
+// applies.  FP64 and
 // complex: tensor-core rows, whose cost goes with the number of m8n8k4 steps
 // (32 values each, however few a block fills), except on small blocks where
 // the pipelined kernel, whose cost goes with the values, fills whole warps
@@ -1606,7 +1612,11 @@ static int fwd_choice(const vbg_matrix* m, bool f32, const ApplyArgs& a, const T
       tiles = tile_use<float, 4, 4>(m, false, a, s, true, &tp) || tile_use<float, 4, 8>(m, false, a, s, true, &tp);
     else
       tiles = tile_use<T>(m, false, a, s, true, &tp);
-    choice = tiles && tp->rows >= 8 ? VBG_KERNEL_TILE : untiled_choice<T>(m, a, s);
+    // FP32: tiles of any height, which the planner then stages one at a time
+    // (us a step at 16 / 32 columns, tiles of 4 rows / pipelined: 5000 rows of
+    // random 4-8 blocks 21 / 68 and 27 / 107, of 1-2 16 / 25 and 17 / 32;
+    // 20000 of 3-5 58 / 75 and 67 / 95, of 8 89 / 103 and 130 / 145)
+    choice = tiles && (narrow || tp->rows >= 8) ? VBG_KERNEL_TILE : untiled_choice<T>(m, a, s);
   } else if ((rc = autotune_fwd<T>(m, a, v, s, &choice))) {
     return rc;
   }

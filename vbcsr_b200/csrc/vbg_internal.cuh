@@ -169,6 +169,7 @@ int reserve_pool(size_t bytes);
 // kernel-layout values are staged in shared memory together.
 struct TilePlan {
   int rows = 0;       // block rows per tile (= warps of the CTA)
+  int stages = 1;     // narrow FP32 rows: tiles staged at a time
   int ntiles = 0;
   int xcap = 0;       // staged X rows of the largest tile
   int owncap = 0;     // scalar rows of the largest tile

@@ -56,16 +56,19 @@ __host__ __device__ inline size_t tile_smem_bytes(int64_t vcap, int ves, int qca
   return 16 + tile_vals_bytes(vcap, ves) + (size_t)qcap + (size_t)xcap * rb;
 }
 
-// Narrow FP32 rows (16 and 32 columns) run on apply_narrow_kernel, which stages
-// the next tile while it multiplies one: two stages of {tile record, row
-// records, values, q-list, X rows}.
+// Narrow FP32 rows (16 and 32 columns) run on apply_narrow_kernel: one or two
+// stages of {tile record, row records, values, q-list, X rows}.  With two the
+// next tile is staged while one is multiplied, where tiles of at least
+// kNarrowTwoRows block rows leave room for that.  Shorter tiles re-read more of
+// X than the overlap hides, so they keep one stage and twice the room.
 __host__ __device__ inline bool tile_narrow(int rb, int ves) { return ves == 4 && rb <= 128; }
 constexpr int kNarrowHead = 64 + kTileRowsMax * 16;  // records of a stage
 __host__ __device__ inline size_t narrow_stage_bytes(int64_t vcap, int qcap, int xcap, int rb) {
   return (size_t)kNarrowHead + tile_vals_bytes(vcap, 4) + (size_t)qcap + (size_t)xcap * rb;
 }
-__host__ __device__ inline size_t tile_plan_smem(int64_t vcap, int ves, int qcap, int xcap, int rb) {
-  return tile_narrow(rb, ves) ? 16 + 2 * narrow_stage_bytes(vcap, qcap, xcap, rb)
+constexpr int kNarrowTwoRows = 8;
+__host__ __device__ inline size_t tile_plan_smem(int64_t vcap, int ves, int qcap, int xcap, int rb, int stages) {
+  return tile_narrow(rb, ves) ? 16 + stages * narrow_stage_bytes(vcap, qcap, xcap, rb)
                               : tile_smem_bytes(vcap, ves, qcap, xcap, rb);
 }
 
@@ -183,9 +186,12 @@ static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, Tile
   auto plan = std::make_unique<TilePlan>();
   int tag = 0;
   // the tallest tile (at most `cap` block rows) whose largest staging fits
-  // the budget
-  for (int tr : {16, 12, 10, 8, 6, 4}) {
-    if (tr > cap) continue;
+  // the budget; narrow FP32 rows: in two stages, else in one
+  std::vector<std::pair<int, int>> heights;
+  for (int stages = tile_narrow(rb, ves) ? 2 : 1; stages >= 1; --stages)
+    for (int tr : {16, 12, 10, 8, 6, 4})
+      if (tr <= cap && (stages == 1 || tr >= kNarrowTwoRows)) heights.emplace_back(tr, stages);
+  for (auto [tr, stages] : heights) {
     bool fits = true;
     int64_t xcap = 0, vcap = 0, ocap = 0;
     int qcap = 0;
@@ -200,10 +206,11 @@ static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, Tile
       qcap = std::max(qcap, qlist_bytes(qstart, t0, t1));
       // shared-memory rows are 16-bit q-list entries
       fits = (int)ranges.size() <= kTileMaxRanges && xcap <= 65535 &&
-             tile_plan_smem(vcap, ves, qcap, (int)xcap, rb) <= (ves == 4 ? kTileSmemBudget32 : kTileSmemBudget);
+             tile_plan_smem(vcap, ves, qcap, (int)xcap, rb, stages) <= (ves == 4 ? kTileSmemBudget32 : kTileSmemBudget);
     }
     if (fits) {
       plan->rows = tr;
+      plan->stages = stages;
       plan->xcap = (int)xcap;
       plan->vcap = vcap;
       plan->owncap = (int)ocap;
@@ -280,7 +287,7 @@ static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, Tile
     k0 += vs;
   }
   plan->ntiles = ntiles;
-  plan->smem = (int)tile_plan_smem(plan->vcap, ves, plan->qcap, plan->xcap, rb);
+  plan->smem = (int)tile_plan_smem(plan->vcap, ves, plan->qcap, plan->xcap, rb, plan->stages);
   if ((rc = plan->tiles.ensure(h_tiles.size() * sizeof(int4), s))) return rc;
   if ((rc = plan->ranges.ensure(std::max<size_t>(h_ranges.size(), 1) * sizeof(int4), s))) return rc;
   if ((rc = plan->xrows.ensure(std::max<size_t>(h_xrows.size(), 1) * sizeof(int), s))) return rc;
@@ -708,12 +715,15 @@ __global__ void __launch_bounds__(kTileWarps * 32, TileMinCtas<T>::v)
 }
 
 // The tiled apply of narrow FP32 multivectors: persistent CTAs over the tiles in
-// a fixed stride, two stages.  Warp 0 issues the next tile's copies (a lane
-// per range of X) before it multiplies its share of this one, so that the
-// copies' latency is behind a tile's work; with one stage the warps waited
-// for it at every tile (4 of 9 cycles between issues at the barrier).  The
-// tile's and the rows' records come with the copies.
-template <int G>
+// a fixed stride, S stages.  With two, warp 0 issues the next tile's copies (a
+// lane per range of X) before it multiplies its share of this one, so that the
+// copies' latency is behind a tile's work; with one the warps wait for it at
+// every tile (4 of 9 cycles between issues at the barrier).  The tile's and the
+// rows' records come with the copies.  One stage, tiles of 4 rows, 5000 block
+// rows of random 4-8 blocks: 21 us at 16 columns and 27 at 32 (with one column
+// a lane and two groups 40 and 46); tiles of 12 rows, 20000 banded block rows
+// of 4-8, 16 columns: 37 (59).
+template <int G, int S>
 __global__ void __launch_bounds__(kTileWarps * 32, 3)
     apply_narrow_kernel(ApplyArgs a, const float* __restrict__ vals, const int4* __restrict__ tiles,
                         const int4* __restrict__ ranges, const unsigned short* __restrict__ qidx,
@@ -738,8 +748,9 @@ __global__ void __launch_bounds__(kTileWarps * 32, 3)
     rc = tiles[4 * (size_t)t + 2];
     rq = tiles[4 * (size_t)t + 3];
   };
-  auto issue = [&](int t, int k) {  // warp 0: tile t (record fetched) into stage k & 1
-    const unsigned st = bar0 + 16 + (unsigned)(k & 1) * stage_bytes, bar = bar0 + 8 * (k & 1);
+  auto issue = [&](int t, int k) {  // warp 0: tile t (record fetched) into stage k mod S
+    const int sg = k & (S - 1);
+    const unsigned st = bar0 + 16 + (unsigned)sg * stage_bytes, bar = bar0 + 8 * sg;
     // the stage's earlier shared-memory reads come before these copies
     fence_proxy_async();
     if (lane == 0) {
@@ -771,18 +782,22 @@ __global__ void __launch_bounds__(kTileWarps * 32, 3)
   }
   bool failed = false;
   for (int k = 0; tile < ntiles; ++k, tile += stride) {
-    if (warp == 0 && tile + stride < ntiles) {
-      issue(tile + stride, k + 1);
-      if (tile + 2 * stride < ntiles) fetch(tile + 2 * stride);
-    }
-    const unsigned bar = bar0 + 8 * (k & 1), parity = (unsigned)(k >> 1) & 1u;
+    auto next = [&]() {
+      if (warp == 0 && tile + stride < ntiles) {
+        issue(tile + stride, k + 1);
+        if (tile + 2 * stride < ntiles) fetch(tile + 2 * stride);
+      }
+    };
+    if (S == 2) next();
+    const int sg = k & (S - 1);
+    const unsigned bar = bar0 + 8 * sg, parity = (unsigned)(k / S) & 1u;
     const bool ok = warp == 0 ? pipe_wait(bar, parity) : true;
     if (!__syncthreads_and(ok)) {
       failed = true;
       break;
     }
     (void)mbar_try_wait(bar, parity);
-    const unsigned char* st = tile_smem + 16 + (size_t)(k & 1) * stage_bytes;
+    const unsigned char* st = tile_smem + 16 + (size_t)sg * stage_bytes;
     const int4* rec = reinterpret_cast<const int4*>(st);
     const int4* rows = reinterpret_cast<const int4*>(st + 64);
     const float* vs = reinterpret_cast<const float*>(st + kNarrowHead);
@@ -806,6 +821,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 3)
       }
     }
     __syncthreads();  // every warp is done with the stage before it is filled again
+    if (S == 1) next();
   }
   if (failed && warp == 0) {
     if (lane == 0) atomicOr(&g_pipe_status, 1u);
@@ -813,8 +829,10 @@ __global__ void __launch_bounds__(kTileWarps * 32, 3)
     // armed again has completed its phase)
     mbar_wait_bounded(bar0, 0u);
     mbar_wait_bounded(bar0, 1u);
-    mbar_wait_bounded(bar0 + 8, 0u);
-    mbar_wait_bounded(bar0 + 8, 1u);
+    if (S == 2) {
+      mbar_wait_bounded(bar0 + 8, 0u);
+      mbar_wait_bounded(bar0 + 8, 1u);
+    }
   }
   if (a.want_dots && !a.row_dots) grid_reduce2(d0, d1, a.partials, a.counter, a.dots_out, part_base, total);
 }
