@@ -162,7 +162,11 @@ int vbg_spmm(const vbg_matrix* m, int k, int ld, const void* X, void* Y, void* s
 #define VBG_KERNEL_TILE 3   /* a CTA per tile of block rows, X ranges staged once per tile */
 #define VBG_KERNEL_CHAIN 4  /* tiles chained per persistent CTA, X rows cached across tiles */
 #define VBG_KERNEL_SCALAR_ROWS 5 /* ld == 1: 1-8 threads per scalar row, the row's blocks split among them */
+#define VBG_KERNEL_LANE_ROWS 6 /* a warp per block row, lanes over the columns of X, scalar multiply-adds */
 int vbg_apply_kernel(const vbg_matrix* m, int ld, int precision, int* kernel);
+/* The same for the adjoint of multivectors (VBG_KERNEL_ROWS or _LANE_ROWS; no
+ * counterpart in the reference). */
+int vbg_adjoint_kernel(const vbg_matrix* m, int ld, int* kernel);
 /* Block rows per tile of the tiled kernel's plan for applies at this leading
  * dimension and precision (no counterpart in the reference): the height the
  * autotuner kept (of tiles of at most 16, 12 and 8 block rows), or the

@@ -1,0 +1,75 @@
+"""Small FP64 and complex blocks in multivector applies: where the scalar rows run
+instead of the tensor-core rows, forward (rows no staged kernel takes) and
+adjoint, on both sides of the rule's lines, with the fused epilogue, against
+the oracle's apply.  Tolerance 1e-12 of the largest value: sums of at most 21
+blocks of 5 products, 110 roundings of 1.1e-16."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from vbcsr_b200 import workloads as W
+
+from .conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def _step(oracle, H, k, adjoint):
+    import torch
+
+    from vbcsr_b200 import _capi
+
+    from . import _gpu
+
+    cplx = np.iscomplexobj(H.values)
+    rng = np.random.default_rng(k)
+    X, P, D, A = (rng.normal(size=(H.N, k)) + (1j * rng.normal(size=(H.N, k)) if cplx else 0) for _ in range(4))
+    dm = _gpu.dmat(H)
+    x, p, d, acc = (_gpu.to_dev_mv(v, k, H.values.dtype) for v in (X, P, D, A))
+    y = torch.zeros_like(x)
+    dots = torch.zeros(2, dtype=torch.float64, device="cuda")
+    ptr = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    c = 0.4 - 0.2j if cplx else 0.4
+    _capi.call("vbg_cheb_step_adjoint" if adjoint else "vbg_cheb_step", dm.h, k, k, 1.7, -0.3, -1.0, ptr(x), ptr(p),
+               ptr(y), ptr(d), ptr(dots), ptr(acc), float(np.real(c)), float(np.imag(c)), None)
+    torch.cuda.synchronize()
+    Y = 1.7 * oracle.apply(H, X, adjoint) - 0.3 * X - P
+    assert rel_err(y.cpu().numpy(), Y) < 1e-12
+    assert rel_err(acc.cpu().numpy(), A + c * Y) < 1e-12
+    ref = np.array([np.sum((D.conj() * Y).real), np.sum(np.abs(Y) ** 2)])
+    assert np.abs(dots.cpu().numpy() - ref).max() < 1e-12 * np.sum(np.abs(D) * np.abs(Y) + np.abs(Y) ** 2)
+    return _capi.adjoint_kernel(dm, k) if adjoint else _capi.apply_kernel(dm, k)
+
+
+def _phases(H, seed):
+    H.values = H.values * np.exp(2j * np.pi * np.random.default_rng(seed).random(H.nnz))
+    return H
+
+
+@pytest.mark.parametrize("cplx,k", [(False, 8), (False, 24), (False, 48), (False, 128), (True, 4), (True, 16), (True, 40)])
+@pytest.mark.parametrize("n,lo,hi", [(1200, 1, 1), (1199, 1, 1), (3600, 1, 3), (3599, 1, 3), (2500, 3, 3)])
+def test_adjoint(oracle, dev, cplx, k, n, lo, hi):
+    H = W.random_pattern(n, lo, hi, 4, seed=n)
+    if cplx:
+        _phases(H, n)
+    # 24 real and 40 complex columns leave many lanes idle
+    want = "lane_rows" if n == 1200 or (n == 3600 and k not in (24, 40)) else "rows"
+    assert _step(oracle, H, k, True) == want
+
+
+@pytest.mark.parametrize("cplx,k", [(False, 8), (False, 48), (False, 128), (True, 4)])
+@pytest.mark.parametrize("n,lo,hi", [(2400, 1, 2), (2399, 1, 2)])
+def test_forward(oracle, dev, cplx, k, n, lo, hi):
+    H = W.random_pattern(n, lo, hi, 40, seed=n)
+    if cplx:
+        _phases(H, n)
+    # (rows of a multiple of 512 bytes: the pipelined kernel)
+    want = "pipe" if k == 128 else "lane_rows" if n == 2400 else "rows"
+    assert _step(oracle, H, k, False) == want
+
+
+@pytest.mark.parametrize("k,want", [(4, "lane_rows"), (8, "rows"), (24, "lane_rows"), (48, "rows"), (32, "lane_rows"), (64, "lane_rows")])
+def test_complex_adjoint_on_many_rows(oracle, dev, k, want):
+    H = _phases(W.tmd_lattice(52, seed=1)[0], 5)  # 8112 block rows of 3 and 5, mean 14.3 values a block
+    assert _step(oracle, H, k, True) == want

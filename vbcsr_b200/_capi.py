@@ -39,6 +39,7 @@ _SIGNATURES = {
     "vbg_memory_reserve": ([C.c_size_t], _i),
     "vbg_memory_trim": ([], _i),
     "vbg_apply_kernel": ([_vp, _i, _i, _pi], _i),
+    "vbg_adjoint_kernel": ([_vp, _i, _pi], _i),
     "vbg_matrix_create": ([C.POINTER(_vp), _i, _i, _pi, _pi, _pi, _vp, _vp], _i),
     "vbg_matrix_destroy": ([_vp], _i),
     "vbg_matrix_duplicate": ([_vp, C.POINTER(_vp), _vp], _i),
@@ -139,14 +140,23 @@ def device_status(clear: bool = True) -> int:
     return int(st.value)
 
 
-KERNEL_NAMES = {0: "vector", 1: "rows", 2: "pipe", 3: "tile", 4: "chain", 5: "scalar_rows"}
+KERNEL_NAMES = {0: "vector", 1: "rows", 2: "pipe", 3: "tile", 4: "chain", 5: "scalar_rows", 6: "lane_rows"}
 
 
 def apply_kernel(dm: "DeviceMatrix", ld: int, precision: int = 0) -> str:
     """Which forward apply kernel this matrix uses at leading dimension ld:
-    'vector' or 'scalar_rows' (ld 1), 'rows', 'pipe', 'tile' or 'chain'."""
+    'vector' or 'scalar_rows' (ld 1), 'rows', 'lane_rows', 'pipe', 'tile' or
+    'chain'."""
     out = C.c_int(-1)
     call("vbg_apply_kernel", dm.h, int(ld), int(precision), C.byref(out))
+    return KERNEL_NAMES[out.value]
+
+
+def adjoint_kernel(dm: "DeviceMatrix", ld: int) -> str:
+    """Which adjoint multivector kernel this matrix uses at leading dimension
+    ld: 'rows' or 'lane_rows'."""
+    out = C.c_int(-1)
+    call("vbg_adjoint_kernel", dm.h, int(ld), C.byref(out))
     return KERNEL_NAMES[out.value]
 
 

@@ -318,9 +318,9 @@ __device__ __forceinline__ bool dispatch_vec_row_meta(const ApplyArgs& a, const 
 // lanes [grp*LPR, grp*LPR + LPR) cover 16-byte vectors of the padded X row;
 // the G lane groups take every G-th block of the row and are summed by
 // butterfly shuffles at the end.  RM output rows per pass (R <= 8 exact).
-template <typename T, int RM>
+template <typename T, int RM, bool ADJ>
 __device__ __forceinline__ void mv_rows(const ApplyArgs& a, const T* __restrict__ vals, int row, int lane, int lpr,
-                                        int G, int o0, int rcount, double& d0, double& d1) {
+                                        int G, int o0, int rcount, int rfull, double& d0, double& d1) {
   constexpr int E = VT<T>::E;
   const int grp = lane / lpr;
   const int vl = lane - grp * lpr;
@@ -340,13 +340,14 @@ __device__ __forceinline__ void mv_rows(const ApplyArgs& a, const T* __restrict_
         const int src = a.ent_src[e];
         const int inner = a.bsz[src];
         const int64_t xrow0 = a.scal_off[src];
-        const T* ab = vals + a.blk_off[e];
+        const T* ab = vals + a.blk_off[ADJ ? a.ent_slot[e] : e];
         for (int q = 0; q < inner; ++q) {
           const Vec<T> xv = load_vec(X, (xrow0 + q) * nvec + vi);
 #pragma unroll
           for (int o = 0; o < RM; ++o) {
             if (o < rcount) {
-              const T av = ab[(int64_t)(o0 + o) * inner + q];
+              T av = ab[ADJ ? (int64_t)q * rfull + o0 + o : (int64_t)(o0 + o) * inner + q];
+              if (ADJ) av = conj_s(av);
 #pragma unroll
               for (int u = 0; u < E; ++u) acc[o].v[u] = fma_s(av, xv.v[u], acc[o].v[u]);
             }
@@ -489,10 +490,10 @@ __global__ void __launch_bounds__(kThreads, 2) apply_vec_wide_kernel(ApplyArgs a
   if (a.want_dots) grid_reduce2(d0, d1, a.partials, a.counter, a.dots_out, part_base, total);
 }
 
-// FP32 multivectors the staged applies do not take: one launch per block-size
-// class; rows [w0, w1) of the class-ordered row list all have block size R
-// (R == 0: any size > 8).  FP64 and complex values run on vbg_mma.cu instead.
-template <typename T, int R>
+// Multivectors the staged applies do not take, FP32 and (lane_rows) small FP64
+// and complex blocks: one launch per block-size class; rows [w0, w1) of the
+// class-ordered row list all have block size R (R == 0: any size > 8).
+template <typename T, int R, bool ADJ>
 __global__ void __launch_bounds__(kThreads) apply_mv_kernel(ApplyArgs a, const T* __restrict__ vals, int w0, int w1,
                                                             int lpr, int G, int part_base, int total) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -501,11 +502,11 @@ __global__ void __launch_bounds__(kThreads) apply_mv_kernel(ApplyArgs a, const T
     const int row = a.order[w];
     double r0 = 0.0, r1 = 0.0;
     if constexpr (R > 0) {
-      mv_rows<T, R>(a, vals, row, lane, lpr, G, 0, R, r0, r1);
+      mv_rows<T, R, ADJ>(a, vals, row, lane, lpr, G, 0, R, R, r0, r1);
     } else {
       const int r = a.bsz[row];
       for (int o0 = 0; o0 < r; o0 += 8)
-        mv_rows<T, 8>(a, vals, row, lane, lpr, G, o0, min(8, r - o0), r0, r1);
+        mv_rows<T, 8, ADJ>(a, vals, row, lane, lpr, G, o0, min(8, r - o0), r, r0, r1);
     }
     if (a.want_dots) {
       if (a.row_dots) {
@@ -700,13 +701,13 @@ static int vec_wide_max_grid() {
   return cached[dev];
 }
 
-template <typename T, int R>
+template <typename T, int R, bool ADJ>
 static int mv_max_grid() {
   static int cached[kMaxDevices] = {};
   const int dev = current_device();
   if (!cached[dev]) {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, apply_mv_kernel<T, R>, kThreads, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, apply_mv_kernel<T, R, ADJ>, kThreads, 0) !=
             cudaSuccess ||
         per_sm < 1)
       per_sm = 1;
@@ -980,32 +981,32 @@ static int launch_vec_t(const vbg_matrix* m, const ApplyArgs& a0, const T* vals,
   return 0;
 }
 
-template <typename T, int R>
+template <typename T, int R, bool ADJ>
 static int launch_mv_class(const ApplyArgs& a, const T* vals, int w0, int w1, int lpr, int G, int grid, int base,
                            int total, cudaStream_t s) {
-  apply_mv_kernel<T, R><<<grid, kThreads, 0, s>>>(a, vals, w0, w1, lpr, G, base, total);
+  apply_mv_kernel<T, R, ADJ><<<grid, kThreads, 0, s>>>(a, vals, w0, w1, lpr, G, base, total);
   VBG_CUDA(cudaGetLastError());
   return 0;
 }
 
-template <typename T>
+template <typename T, bool ADJ>
 static int mv_class_grid(int r, int rows) {
   int cap;
   switch (r) {
-    case 1: cap = mv_max_grid<T, 1>(); break;
-    case 2: cap = mv_max_grid<T, 2>(); break;
-    case 3: cap = mv_max_grid<T, 3>(); break;
-    case 4: cap = mv_max_grid<T, 4>(); break;
-    case 5: cap = mv_max_grid<T, 5>(); break;
-    case 6: cap = mv_max_grid<T, 6>(); break;
-    case 7: cap = mv_max_grid<T, 7>(); break;
-    case 8: cap = mv_max_grid<T, 8>(); break;
-    default: cap = mv_max_grid<T, 0>(); break;
+    case 1: cap = mv_max_grid<T, 1, ADJ>(); break;
+    case 2: cap = mv_max_grid<T, 2, ADJ>(); break;
+    case 3: cap = mv_max_grid<T, 3, ADJ>(); break;
+    case 4: cap = mv_max_grid<T, 4, ADJ>(); break;
+    case 5: cap = mv_max_grid<T, 5, ADJ>(); break;
+    case 6: cap = mv_max_grid<T, 6, ADJ>(); break;
+    case 7: cap = mv_max_grid<T, 7, ADJ>(); break;
+    case 8: cap = mv_max_grid<T, 8, ADJ>(); break;
+    default: cap = mv_max_grid<T, 0, ADJ>(); break;
   }
   return std::max(1, std::min((rows + kWarps - 1) / kWarps, cap));
 }
 
-template <typename T>
+template <typename T, bool ADJ>
 static int launch_mv_t(const vbg_matrix* m, const ApplyArgs& a, const T* vals, cudaStream_t s) {
   const int nvec = a.ld / VT<T>::E;
   int lpr = nvec >= 32 ? 32 : nvec;
@@ -1023,7 +1024,7 @@ static int launch_mv_t(const vbg_matrix* m, const ApplyArgs& a, const T* vals, c
   std::vector<int> grids;
   int total = 0;
   for (auto& sg : segs) {
-    grids.push_back(mv_class_grid<T>(std::get<0>(sg), std::get<2>(sg) - std::get<1>(sg)));
+    grids.push_back(mv_class_grid<T, ADJ>(std::get<0>(sg), std::get<2>(sg) - std::get<1>(sg)));
     total += grids.back();
   }
   if (int rc = check_dot_ctas(a, total)) return rc;
@@ -1032,15 +1033,15 @@ static int launch_mv_t(const vbg_matrix* m, const ApplyArgs& a, const T* vals, c
     const int w0 = std::get<1>(segs[i]), w1 = std::get<2>(segs[i]);
     int rc = 0;
     switch (std::get<0>(segs[i])) {
-      case 1: rc = launch_mv_class<T, 1>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      case 2: rc = launch_mv_class<T, 2>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      case 3: rc = launch_mv_class<T, 3>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      case 4: rc = launch_mv_class<T, 4>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      case 5: rc = launch_mv_class<T, 5>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      case 6: rc = launch_mv_class<T, 6>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      case 7: rc = launch_mv_class<T, 7>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      case 8: rc = launch_mv_class<T, 8>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
-      default: rc = launch_mv_class<T, 0>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 1: rc = launch_mv_class<T, 1, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 2: rc = launch_mv_class<T, 2, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 3: rc = launch_mv_class<T, 3, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 4: rc = launch_mv_class<T, 4, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 5: rc = launch_mv_class<T, 5, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 6: rc = launch_mv_class<T, 6, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 7: rc = launch_mv_class<T, 7, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      case 8: rc = launch_mv_class<T, 8, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
+      default: rc = launch_mv_class<T, 0, ADJ>(a, vals, w0, w1, lpr, G, grids[i], base, total, s); break;
     }
     if (rc) return rc;
     base += grids[i];
@@ -1422,9 +1423,40 @@ static int prepare(const vbg_matrix* m, bool adj, int k, int ld, ApplyArgs& a, c
   return 0;
 }
 
-// Forward multivector apply on kernel `which` (VBG_KERNEL_CHAIN, _TILE, _PIPE
-// or _ROWS; -1: the default order -- chained tiles when the apply.chain
-// option allows them, tiles, the pipelined kernel, rows).  Returns
+// Whether rows of FP64 or complex values run on apply_mv_kernel instead of the
+// tensor-core rows of vbg_mma.cu (the adjoint, and forward what no staged
+// apply takes).  A tensor-core step holds 32 values however few a block fills,
+// while a warp here spends its lanes on columns and its lane groups on several
+// blocks, but the block sizes' launches follow one another.  So: blocks of at
+// most 7 values on average, with at least 1200 block rows a size, unless the
+// columns leave over a quarter of the lanes idle (nvec 16-byte vectors a row;
+// lane groups need a power of two below 32) and the blocks are not single
+// values (20000 rows, real 24 columns: sizes 1-2 68 / 66, 1 66 / 50).  And complex adjoints of larger small blocks,
+// whose steps are four real ones, on many rows: whole warps of columns, or so
+// few that the groups take several blocks (4 columns), or 24.
+// us an apply, tensor-core rows / these (20000 random block rows of 13 blocks,
+// adjoint): sizes 1-2 real 8 columns 58 / 29, 64 columns 140 / 89, complex 16
+// columns 105 / 55; sizes 2-3 74 real 32 columns / 61; sizes 2-4 (mean 9) real
+// 16 columns 60 / 84, complex 64 columns 472 / 443; 60000 banded rows of 1-3,
+// complex 128 columns 2890 / 985.  5000 rows of 1-2: real 8 columns 23 / 17,
+// 32 columns 23 / 25; 1500 rows of 1-2, real 32 columns 15 / 26.  120000 rows
+// of 3 and 5, complex adjoint, 4 / 16 / 64 columns 480 / 624 / 2513 against
+// 428 / 800 / 1840.
+template <typename T>
+static bool lane_rows(const vbg_matrix* m, const ApplyArgs& a, bool adj) {
+  constexpr bool cx = std::is_same<T, cplx>::value;
+  // (a caller's own dot scratch is sized for the single launch)
+  if (std::is_same<T, float>::value || a.max_ctas > 0 || m->nnzb == 0) return false;
+  const int nvec = a.ld / VT<T>::E;
+  const bool lanes = nvec < 24 ? (nvec & (nvec - 1)) == 0 : 4 * nvec >= 3 * ((nvec + 31) / 32 * 32);
+  const double mean = (double)m->nnz / (double)m->nnzb;
+  if (mean <= (lanes ? 7.0 : 1.5) && m->n >= 1200 * (int64_t)m->class_segs.size()) return true;
+  return cx && adj && mean <= 15.0 && m->n >= 8000 && (nvec <= 4 || nvec == 24 || nvec % 32 == 0);
+}
+
+// Forward multivector apply on kernel `which` (VBG_KERNEL_CHAIN, _TILE, _PIPE,
+// _ROWS or _LANE_ROWS; -1: the default order -- chained tiles when the
+// apply.chain option allows them, tiles, the pipelined kernel, rows).  Returns
 // kNotApplicable when `which` cannot run this apply.
 constexpr int kNotApplicable = 1;
 
@@ -1459,7 +1491,8 @@ static int launch_fwd_mv(const vbg_matrix* m, const ApplyArgs& a, const T* v, cu
     if (pipe_use<T>(m, false, a, s, allow_alloc)) return launch_pipe_t<T>(m, a, s);
     if (!any) return kNotApplicable;
   }
-  if constexpr (std::is_same<T, float>::value) return launch_mv_t<float>(m, a, v, s);
+  if constexpr (std::is_same<T, float>::value) return launch_mv_t<float, false>(m, a, v, s);
+  if (which == VBG_KERNEL_LANE_ROWS || (any && lane_rows<T>(m, a, false))) return launch_mv_t<T, false>(m, a, v, s);
   return launch_mma(m, false, a, s);
 }
 
@@ -1481,7 +1514,8 @@ static int untiled_choice(const vbg_matrix* m, const ApplyArgs& a, cudaStream_t 
   const bool full = (int64_t)a.ld * (int)sizeof(T) % 512 == 0;
   const double most = full ? 20.0 : cx ? 10.0 : 0.0;
   const bool pipe = f32 || (double)m->nnz <= most * (double)m->nnzb;
-  return pipe && pipe_use<T>(m, false, a, s, true) ? VBG_KERNEL_PIPE : VBG_KERNEL_ROWS;
+  if (pipe && pipe_use<T>(m, false, a, s, true)) return VBG_KERNEL_PIPE;
+  return lane_rows<T>(m, a, false) ? VBG_KERNEL_LANE_ROWS : VBG_KERNEL_ROWS;
 }
 
 // The autotuner: the first forward multivector apply with a given leading
@@ -1752,11 +1786,13 @@ static int launch_apply(const vbg_matrix* m, bool adj, bool f32, const ApplyArgs
   }
   if (m->dtype == VBG_C128) {
     const cplx* v = m->vals.as<cplx>();
-    if (adj) return mv ? launch_mma(m, true, a, s) : launch_vec_t<cplx, true>(m, a, v, s);
+    if (adj && mv) return lane_rows<cplx>(m, a, true) ? launch_mv_t<cplx, true>(m, a, v, s) : launch_mma(m, true, a, s);
+    if (adj) return launch_vec_t<cplx, true>(m, a, v, s);
     return mv ? fwd(cplx{}, v) : launch_vec_t<cplx, false>(m, a, v, s);
   }
   const double* v = m->vals.as<double>();
-  if (adj) return mv ? launch_mma(m, true, a, s) : launch_vec_t<double, true>(m, a, v, s);
+  if (adj && mv) return lane_rows<double>(m, a, true) ? launch_mv_t<double, true>(m, a, v, s) : launch_mma(m, true, a, s);
+  if (adj) return launch_vec_t<double, true>(m, a, v, s);
   return mv ? fwd(double{}, v) : launch_vec_t<double, false>(m, a, v, s);
 }
 
@@ -2143,7 +2179,24 @@ int vbg_apply_kernel(const vbg_matrix* m, int ld, int precision, int* kernel) {
     tile = chain || tile_use<double>(m, false, a, nullptr, true, &tp);
     pipe = tile || pipe_use<double>(m, false, a, nullptr, true);
   }
-  *kernel = chain ? VBG_KERNEL_CHAIN : tile ? VBG_KERNEL_TILE : pipe ? VBG_KERNEL_PIPE : VBG_KERNEL_ROWS;
+  const bool lane = m->dtype == VBG_C128 ? lane_rows<cplx>(m, a, false)
+                                         : precision == VBG_PREC_F64 && lane_rows<double>(m, a, false);
+  *kernel = chain ? VBG_KERNEL_CHAIN
+            : tile ? VBG_KERNEL_TILE
+            : pipe ? VBG_KERNEL_PIPE
+            : lane ? VBG_KERNEL_LANE_ROWS
+                   : VBG_KERNEL_ROWS;
+  return 0;
+}
+
+int vbg_adjoint_kernel(const vbg_matrix* m, int ld, int* kernel) {
+  VBG_CHECK(m && kernel, VBG_E_ARG, "null argument");
+  VBG_CHECK(ld > 1, VBG_E_ARG, "the adjoint of multivectors only (ld > 1)");
+  ApplyArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.ld = ld;
+  const bool lane = m->dtype == VBG_C128 ? lane_rows<cplx>(m, a, true) : lane_rows<double>(m, a, true);
+  *kernel = lane ? VBG_KERNEL_LANE_ROWS : VBG_KERNEL_ROWS;
   return 0;
 }
 
