@@ -50,3 +50,19 @@ def test_wide_vector(oracle, dev, name, cplx, adjoint):
     assert rel_err(yd.cpu().numpy(), y) < 1e-12
     want = np.array([np.sum((d.conj() * y).real), np.sum(np.abs(y) ** 2)])
     assert np.abs(dots.cpu().numpy() - want).max() < 1e-12 * np.sum(np.abs(d) * np.abs(y) + np.abs(y) ** 2)
+
+
+@pytest.mark.parametrize("name", list(_CASES))
+def test_wide_vector_fp32(oracle, dev, name):
+    """FP32 moments of one vector.  A step's 250 roundings of 6e-8 are 1.5e-5 of
+    an entry at most, the three steps of six moments (1 + 3 + 5) times that,
+    1.4e-4; a moment adds N > 30 entries' errors of either sign over mu_0 = N."""
+    from . import _gpu
+
+    n, lo, hi, per = _CASES[name]
+    H = W.random_pattern(n, lo, hi, per, seed=41)
+    H.values = (H.values - 0.5) / W.gershgorin_bound(H)
+    V = np.where(np.random.default_rng(3).random((H.N, 1)) < 0.5, -1.0, 1.0)
+    mu = _gpu.kpm_moments(_gpu.dmat(H), V, 6, precision=1)
+    ref = oracle.kpm_moments(H, V, 6, True)
+    assert np.abs(mu - ref).max() / abs(ref[0]) < 3e-5
