@@ -1,8 +1,8 @@
 """Small FP64 and complex blocks in multivector applies: where the scalar rows run
 instead of the tensor-core rows, forward (rows no staged kernel takes) and
 adjoint, on both sides of the rule's lines, with the fused epilogue, against
-the oracle's apply.  Tolerance 1e-12 of the largest value: sums of at most 21
-blocks of 5 products, 110 roundings of 1.1e-16."""
+the oracle's apply.  Tolerance 1e-12 of the largest value: sums of at most 41
+blocks of 5 products, 210 roundings of 1.1e-16."""
 import ctypes as C
 
 import numpy as np
@@ -73,3 +73,14 @@ def test_forward(oracle, dev, cplx, k, n, lo, hi):
 def test_complex_adjoint_on_many_rows(oracle, dev, k, want):
     H = _phases(W.tmd_lattice(52, seed=1)[0], 5)  # 8112 block rows of 3 and 5, mean 14.3 values a block
     assert _step(oracle, H, k, True) == want
+
+
+@pytest.mark.parametrize("cplx,k,n,lo,hi,want", [
+    (False, 64, 500, 2, 4, "rows"), (False, 64, 2999, 3, 5, "rows"), (False, 64, 3000, 3, 5, "pipe"),
+    (False, 128, 1500, 2, 4, "pipe"), (True, 32, 2499, 2, 4, "rows"), (True, 64, 1250, 2, 4, "pipe"),
+    (False, 64, 16000, 8, 8, "pipe"), (False, 64, 15999, 8, 8, "rows"), (False, 64, 16000, 7, 8, "rows")])
+def test_rows_of_512_bytes_without_tiles(oracle, dev, cplx, k, n, lo, hi, want):
+    H = W.random_pattern(n, lo, hi, 10 if hi == 8 else 40, seed=n)
+    if cplx:
+        _phases(H, n)
+    assert _step(oracle, H, k, False) == want

@@ -1517,21 +1517,35 @@ static int launch_fwd_mv(const vbg_matrix* m, const ApplyArgs& a, const T* v, cu
 // The kernel of a forward multivector apply whose matrix has no tiles (FP64 and
 // complex: none of at least 8 block rows).  FP32: the pipelined kernel where it
 // applies.  FP64 and
-// complex: tensor-core rows, whose cost goes with the number of m8n8k4 steps
-// (32 values each, however few a block fills), except on small blocks where
-// the pipelined kernel, whose cost goes with the values, fills whole warps
-// (rows of a multiple of 512 bytes), or whose real multiply-adds stand against
-// four steps a product (complex).  By the mean values of a block; us an apply,
-// pipelined / rows, 20000 block rows of 13 random blocks, real 64 columns:
-// sizes 2-4 (mean 9) 98 / 134, 3-5 (16) 109 / 152, 4-8 (36) 389 / 169; real
-// 128 columns 203 / 287, 229 / 311, 560 / 351; complex 16 columns 1-2 (2)
-// 77 / 106, 2-4 105 / 107, 3-5 121 / 117; real 32 columns 74 / 68, 89 / 70.
+// complex: rows (lane_rows or on the tensor cores), except where the pipelined
+// kernel, whose cost goes with the values, is faster.  On rows of a multiple of
+// 512 bytes it fills whole warps: blocks of at most 20 values on average, or
+// many real rows of one block size at 512 bytes, once there are rows enough to
+// fill the SMs with its warps of 512 bytes (3000; complex, whose products are
+// four times the work, 2500).  On other complex rows: blocks of at most 10
+// values, whose products would be four tensor-core steps each.
+// us an apply, pipelined / tensor-core rows, random rows of 13 blocks, real 64
+// columns: 20000 rows of sizes 2-4 (mean 9) 99 / 130, 3-5 (16) 109 / 151, 4-8
+// (36) 412 / 169, 8 (64) 175 / 195; 5000 rows 2-4 36 / 38, 3-5 40 / 40, 8
+// 62 / 54; 1500 rows 2-4 32 / 19; 500 rows 2-4 32 / 11, where tiles of 4 rows
+// took 13.  Real 128 columns, 20000 rows: 203 / 287, 229 / 311, 560 / 351, 8
+// 369 / 345; complex 16 columns 1-2 (2) 77 / 106, 2-4 99 / 107, 3-5 120 / 116,
+// 64 columns 1500 rows 2-4 1.16 of the rows', 5000 0.81.  Real 32 columns 90 / 69,
+// 115 / 75; rows of no multiple of 512 bytes beyond (48, 80, 96, 112, 144 real
+// columns) never were faster pipelined: 20000 rows of 3-5 222 / 136 at 48, 314 /
+// 219 at 96, a lattice of 30000 rows 285 / 189 and 388 / 298.
 template <typename T>
 static int untiled_choice(const vbg_matrix* m, const ApplyArgs& a, cudaStream_t s) {
   constexpr bool f32 = std::is_same<T, float>::value, cx = std::is_same<T, cplx>::value;
-  const bool full = (int64_t)a.ld * (int)sizeof(T) % 512 == 0;
-  const double most = full ? 20.0 : cx ? 10.0 : 0.0;
-  const bool pipe = f32 || (double)m->nnz <= most * (double)m->nnzb;
+  const int64_t bytes = (int64_t)a.ld * (int)sizeof(T);
+  const double mean = m->nnzb ? (double)m->nnz / (double)m->nnzb : 0.0;
+  bool pipe = f32;
+  if (!f32 && bytes % 512 == 0) {
+    const bool enough = m->n * (bytes / 512) >= (cx ? 2500 : 3000);
+    pipe = enough && (mean <= 20.0 || (!cx && bytes == 512 && m->min_bs == m->max_bs && m->n >= 16000));
+  } else if (cx) {
+    pipe = mean <= 10.0;
+  }
   if (pipe && pipe_use<T>(m, false, a, s, true)) return VBG_KERNEL_PIPE;
   return lane_rows<T>(m, a, false) ? VBG_KERNEL_LANE_ROWS : VBG_KERNEL_ROWS;
 }
