@@ -191,15 +191,25 @@ __global__ void __launch_bounds__(kTileWarps * 32, 2)
         return xs_base + (unsigned)slot * RB + (unsigned)dtile_chunk(g, slot) * 16;
       };
       int q = 0;
-#pragma unroll 2
-      for (; q + 4 <= nq; q += 4) {
+      // even and odd steps summed apart: half the chain, and the rounding error
+      // of the two lane groups that this replaced
+      double odd[NP][4] = {};
+      auto step = [&](double (&c)[NP][4], int q) {
         const unsigned char* xr = chunk(ql[q]);
         const T av = va[q * rp];
         double2 b[NP];
 #pragma unroll
         for (int p = 0; p < NP; ++p) b[p] = *reinterpret_cast<const double2*>(xr + 128 * p);
 #pragma unroll
-        for (int p = 0; p < NP; ++p) dtile_mma<T>(acc[p], av, b[p]);
+        for (int p = 0; p < NP; ++p) dtile_mma<T>(c[p], av, b[p]);
+      };
+      for (; q + 8 <= nq; q += 8) {
+        step(acc, q);
+        step(odd, q + 4);
+      }
+      if (q + 4 <= nq) {
+        step(odd, q);
+        q += 4;
       }
       if (q < nq) {  // the last one to three X rows: zero operands beyond them
         const bool kv = q + t4 < nq;
@@ -211,6 +221,10 @@ __global__ void __launch_bounds__(kTileWarps * 32, 2)
           dtile_mma<T>(acc[p], av, b);
         }
       }
+#pragma unroll
+      for (int p = 0; p < NP; ++p)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) acc[p][t] += odd[p][t];
       double rd0 = 0.0, rd1 = 0.0;
       if (g < r) {
         const int oslot = tc.x + (int)(y0 - tc.z) + g;

@@ -128,6 +128,8 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2)
     apply_mma_kernel(ApplyArgs a, const T* __restrict__ vals, int rgroups, int cgroups, int split, int part_base,
                      int total) {
   constexpr int W = std::is_same<T, cplx>::value ? 2 : 1;  // doubles per element
+  // even and odd fragments are summed apart where the registers allow it
+  constexpr bool DUAL = MT * NP == 1;
   extern __shared__ double mma_red[];  // split > 1: kMmaWarps tiles of MT * NP * 4 * 32 doubles
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t4 = lane & 3;
@@ -159,6 +161,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2)
         for (int p = 0; p < NP; ++p)
 #pragma unroll
           for (int t = 0; t < 4; ++t) acc[m][p][t] = 0.0;
+      double odd[DUAL ? MT : 1][DUAL ? NP : 1][4] = {};
       if (o0 < r) {
         for (int base = e0 + sub; base < e1; base += 32 * split) {
           const int cnt = min(32, (e1 - base + split - 1) / split);
@@ -219,10 +222,15 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2)
             if (!more) break;
             more = next();
             if (more) load(f0);
-            mma_step<T, MT, NP>(acc, f1, mlive);
+            if constexpr (DUAL) mma_step<T, MT, NP>(odd, f1, mlive);
+            else mma_step<T, MT, NP>(acc, f1, mlive);
             if (!more) break;
           }
         }
+      }
+      if constexpr (DUAL) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) acc[0][0][t] += odd[0][0][t];
       }
       if (split > 1) {
         double* mine = mma_red + (size_t)warp * (MT * NP * 4 * 32) + lane;
