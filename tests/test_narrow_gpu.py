@@ -177,3 +177,21 @@ def test_tensor_core_tiles_rounding(dev, k):
     rms = lambda a: float(np.sqrt(np.mean((a.astype(np.longdouble) - exact) ** 2)))  # noqa: E731
     assert rms(one) > 1.2 * rms(two)
     assert rms(y) < 1.1 * rms(two)
+
+
+@pytest.mark.parametrize("cplx,k", [(False, 16), (False, 64), (True, 8)])
+def test_short_tiles_are_not_planned(oracle, dev, cplx, k):
+    """Tiles that the choice has no use for (below 8 block rows) are not built."""
+    from vbcsr_b200 import _capi
+
+    from . import _gpu
+
+    H = W.random_pattern(1500, 2, 4, 12, seed=7)
+    if cplx:
+        H.values = H.values * np.exp(2j * np.pi * np.random.default_rng(1).random(H.nnz))
+    rng = np.random.default_rng(k)
+    X = rng.normal(size=(H.N, k)) + (1j * rng.normal(size=(H.N, k)) if cplx else 0)
+    dm = _gpu.dmat(H)
+    assert rel_err(_gpu.apply(dm, X), oracle.apply(H, X)) < 1e-12
+    assert _capi.apply_kernel(dm, k) == ("pipe" if cplx else "rows")
+    assert _capi.apply_tile_rows(dm, k) == 0

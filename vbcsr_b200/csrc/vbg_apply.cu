@@ -23,6 +23,7 @@
 #include <atomic>
 #include <cstring>
 #include <mutex>
+#include <numeric>
 #include <type_traits>
 
 #include "vbg_internal.cuh"
@@ -1211,10 +1212,10 @@ static int dtile_pieces(int ld) {
 // with EV = 4 and G = 4 and 8 lane groups); the pipelined apply's value
 // layout applies, the staged rows (X, Xprev, the dot partner) start on
 // 16-byte boundaries, and the matrix has a tile plan for it (built here
-// unless capturing or allocation is not allowed).
+// unless capturing or allocation is not allowed) of at least `floor` block rows.
 template <typename T, int EV = PipeEV<T>::v, int G = 1>
 static bool tile_use(const vbg_matrix* m, bool adj, const ApplyArgs& a, cudaStream_t s, bool allow_alloc,
-                     TilePlan** plan) {
+                     TilePlan** plan, int floor = 0) {
   *plan = nullptr;
   if (dtile_pieces<T>(a.ld) == 0 && a.ld != 32 / G * EV) return false;
   if (!pipe_use<T>(m, adj, a, s, allow_alloc)) return false;
@@ -1225,13 +1226,13 @@ static bool tile_use(const vbg_matrix* m, bool adj, const ApplyArgs& a, cudaStre
   const int cap = tile_cap(m, a.ld, (int)sizeof(T));
   auto it = m->tile_plans.find(std::make_tuple(rb, (int)sizeof(T), cap));
   if (it != m->tile_plans.end()) {
-    if (it->second->rows > 0) *plan = it->second.get();
+    if (it->second->rows > std::max(floor - 1, 0)) *plan = it->second.get();
     return *plan != nullptr;
   }
   if (!allow_alloc) return false;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return false;
-  return tile_plan(m, rb, (int)sizeof(T), s, plan, cap) == 0 && *plan != nullptr;
+  return tile_plan(m, rb, (int)sizeof(T), s, plan, cap, floor) == 0 && *plan != nullptr;
 }
 
 // Grid of apply_tile_kernel<T, EV, G> for a plan: the CTAs resident at once,
@@ -1591,7 +1592,7 @@ static int autotune_fwd(const vbg_matrix* m, const ApplyArgs& a0, const T* v, cu
   std::vector<int> cands = {VBG_KERNEL_CHAIN, VBG_KERNEL_TILE, VBG_KERNEL_PIPE};
   TilePlan* tp = nullptr;
   if constexpr (!f32) {
-    const bool tiles = tile_use<T>(m, false, a, s, true, &tp) && tp->rows >= 8;
+    const bool tiles = tile_use<T>(m, false, a, s, true, &tp, 8);
     if (tiles) cands = {VBG_KERNEL_CHAIN, VBG_KERNEL_TILE};
     else cands.clear();
   }
@@ -1677,12 +1678,12 @@ static int fwd_choice(const vbg_matrix* m, bool f32, const ApplyArgs& a, const T
     if constexpr (std::is_same<T, float>::value)
       tiles = tile_use<float, 4, 4>(m, false, a, s, true, &tp) || tile_use<float, 4, 8>(m, false, a, s, true, &tp);
     else
-      tiles = tile_use<T>(m, false, a, s, true, &tp);
+      tiles = tile_use<T>(m, false, a, s, true, &tp, 8);
     // FP32: tiles of any height, which the planner then stages one at a time
     // (us a step at 16 / 32 columns, tiles of 4 rows / pipelined: 5000 rows of
     // random 4-8 blocks 21 / 68 and 27 / 107, of 1-2 16 / 25 and 17 / 32;
     // 20000 of 3-5 58 / 75 and 67 / 95, of 8 89 / 103 and 130 / 145)
-    choice = tiles && (narrow || tp->rows >= 8) ? VBG_KERNEL_TILE : untiled_choice<T>(m, a, s);
+    choice = tiles ? VBG_KERNEL_TILE : untiled_choice<T>(m, a, s);
   } else if ((rc = autotune_fwd<T>(m, a, v, s, &choice))) {
     return rc;
   }

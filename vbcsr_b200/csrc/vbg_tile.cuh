@@ -86,18 +86,29 @@ static void balanced_runs(const int64_t* w, int T, int W, int* bounds) {
     cut[1][j] = 0;
   }
   const int K = std::min(W, std::max(T, 1));
-  for (int k = 2; k <= K; ++k)
+  for (int k = 2; k <= K; ++k) {
+    int at = 0;  // the first best cut of the previous j
     for (int j = 0; j <= T; ++j) {
       best[k][j] = best[k - 1][j];
       cut[k][j] = j;
-      for (int i = 0; i < j; ++i) {
+      // the larger of a rising and a falling sequence in i: the best cut moves
+      // right with j (by one to the left at most), and past the point where the
+      // rising one leads nothing is better
+      int64_t least = INT64_MAX;
+      for (int i = std::max(0, at - 1); i < j; ++i) {
         const int64_t v = std::max(best[k - 1][i], pre[j] - pre[i]);
-        if (v < best[k][j]) {
-          best[k][j] = v;
-          cut[k][j] = i;
+        if (v < least) {
+          least = v;
+          at = i;
         }
+        if (best[k - 1][i] >= least) break;
+      }
+      if (least < best[k][j]) {
+        best[k][j] = least;
+        cut[k][j] = at;
       }
     }
+  }
   int end = T;
   for (int k = K; k >= 1; --k) {
     bounds[k - 1] = end;
@@ -128,17 +139,19 @@ static inline int qlist_bytes(const std::vector<int>& qstart, int t0, int t1) {
 }
 
 // Plans the row tiles of matrix m for X rows of rb bytes and values of ves
-// bytes (kernel layout), tiles of at most `cap` block rows.  *out is the
-// plan, or nullptr when no tile height fits the budget.  Needs the spans (ensure_spans); reads the host
-// structure.
+// bytes (kernel layout), tiles of at most `cap` and at least `floor` block
+// rows.  *out is the plan, or nullptr when no such height fits the budget
+// (remembered unless `floor` is what ruled it out: a caller that has no use for
+// short tiles does not pay for their lists, 65k random blocks in tiles of 4 rows
+// 9 ms).  Needs the spans (ensure_spans); reads the host structure.
 static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, TilePlan** out,
-                     int cap = kTileRowsMax) {
+                     int cap = kTileRowsMax, int floor = 0) {
   auto* m = const_cast<vbg_matrix*>(cm);
   *out = nullptr;
   const auto key = std::make_tuple(rb, ves, cap);
   auto found = m->tile_plans.find(key);
   if (found != m->tile_plans.end()) {
-    if (found->second->rows > 0) *out = found->second.get();
+    if (found->second->rows > std::max(floor - 1, 0)) *out = found->second.get();
     return 0;
   }
   VBG_CHECK(m->span_cap > 0 && (int64_t)m->h_span_x.size() == m->nspans, VBG_E_STATE, "tile plan needs the spans");
@@ -190,7 +203,7 @@ static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, Tile
   std::vector<std::pair<int, int>> heights;
   for (int stages = tile_narrow(rb, ves) ? 2 : 1; stages >= 1; --stages)
     for (int tr : {16, 12, 10, 8, 6, 4})
-      if (tr <= cap && (stages == 1 || tr >= kNarrowTwoRows)) heights.emplace_back(tr, stages);
+      if (tr <= cap && tr >= floor && (stages == 1 || tr >= kNarrowTwoRows)) heights.emplace_back(tr, stages);
   for (auto [tr, stages] : heights) {
     bool fits = true;
     int64_t xcap = 0, vcap = 0, ocap = 0;
@@ -218,6 +231,7 @@ static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, Tile
       break;
     }
   }
+  if (plan->rows == 0 && floor > 0) return 0;
   if (plan->rows == 0) {  // remembered as infeasible
     m->tile_plans[key] = std::move(plan);
     return 0;
@@ -227,6 +241,7 @@ static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, Tile
   std::vector<int4> h_tiles(4 * (size_t)ntiles), h_ranges, h_rowinfo(std::max(n, 1));
   const bool steps = ves > 4 && rb <= 256;  // runs on the tensor-core form (vbg_dtile.cuh)
   std::vector<int> h_xrows;  // of which: the staged X rows one by one
+  std::vector<int> srow(n);  // of the tile at hand: the shared-memory row of a block column's first X row
   // the q-list, padded so that the last tile's staged slice stays inside
   std::vector<unsigned short> h_qidx(((size_t)qstart[n] + 7) / 8 * 8 + 8, 0);
   int64_t k0 = 0;  // kernel-layout value offset of the tile's first slot
@@ -242,19 +257,16 @@ static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, Tile
     }
     const int rend = (int)h_ranges.size();
     const int xoff = (int)h_xrows.size();
-    if (steps)
+    if (steps) {
+      h_xrows.resize((size_t)xoff + dst);
       for (int k = rbeg; k < rend; ++k)
-        for (int x = 0; x < h_ranges[k].y; ++x) h_xrows.push_back(h_ranges[k].x + x);
-    // the shared-memory row of a staged X row
-    auto srow_of = [&](int x) {
-      int lo = rbeg, hi = rend - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) / 2;
-        if (h_ranges[mid].x <= x) lo = mid;
-        else hi = mid - 1;
-      }
-      return h_ranges[lo].z + (x - h_ranges[lo].x);
-    };
+        std::iota(h_xrows.begin() + xoff + h_ranges[k].z, h_xrows.begin() + xoff + h_ranges[k].z + h_ranges[k].y,
+                  h_ranges[k].x);
+    }
+    // the shared-memory row of each block column's first X row
+    for (int g = rbeg; g < rend; ++g)
+      for (int c = ranges[g - rbeg].x; c <= ranges[g - rbeg].y; ++c)
+        srow[c] = h_ranges[g].z + (int)(soff[c] - soff[ranges[g - rbeg].x]);
     // every block row's q-list: the shared-memory row of each X row its
     // blocks read (a block column's rows lie in one range)
     const int qb = qlist_base(qstart, t0);
@@ -262,8 +274,8 @@ static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, Tile
     for (int i = t0; i < t1; ++i) {
       int k = qstart[i];
       for (int p = rp[i]; p < rp[i + 1]; ++p) {
-        const int x0 = (int)soff[ci[p]];
-        for (int q = 0; q < bsz[ci[p]]; ++q) h_qidx[k++] = (unsigned short)srow_of(x0 + q);
+        const int x0 = srow[ci[p]], x1 = x0 + bsz[ci[p]];
+        for (int x = x0; x < x1; ++x) h_qidx[k++] = (unsigned short)x;
       }
       // narrow: the row's first scalar row within the tile beside its size
       h_rowinfo[i] = make_int4(qstart[i] - qb, qn[i], (int)vs,
@@ -282,7 +294,7 @@ static int tile_plan(const vbg_matrix* cm, int rb, int ves, cudaStream_t s, Tile
     const int ys0 = (int)soff[t0], own = (int)(soff[t1] - soff[t0]);
     h_tiles[4 * (size_t)t] = make_int4(t0, t1, rbeg, rend);
     h_tiles[4 * (size_t)t + 1] = make_int4((int)(k0 & 0xffffffff), (int)(k0 >> 32), (int)(vs * ves), dst * rb);
-    h_tiles[4 * (size_t)t + 2] = make_int4(srow_of(ys0), own, ys0, xoff);
+    h_tiles[4 * (size_t)t + 2] = make_int4(srow[t0], own, ys0, xoff);
     h_tiles[4 * (size_t)t + 3] = make_int4(qb, qlist_bytes(qstart, t0, t1), (int)packed[0], (int)packed[1]);
     k0 += vs;
   }
