@@ -230,10 +230,14 @@ int vbg_cheb_series(const vbg_matrix* m, int k, int ld, const void* V, int M, co
  * multivectors of vbg_sddmm.  last / before (may be NULL) receive the last
  * vector and the one before it.  One launch for all steps when the matrix
  * fits the SMs' shared memory (its values at most about 30 MB, blocks at most
- * 8 x 8), as vbg_cheb_series does for vectors. */
+ * 8 x 8) and has run steps enough to repay the plan this takes, as
+ * vbg_cheb_series does for vectors. */
 int vbg_cheb_columns(const vbg_matrix* m, int adjoint, const void* x0, const void* x1, int steps,
                      const double* coeffs, const void* source, void* cols, int64_t ldc, int ncol, int col0, int dcol,
                      void* last, void* before, void* stream);
+/* Whether vector recurrences on m have run as one launch, over A (adjoint 0)
+ * or A^H (no counterpart in the reference). */
+int vbg_recurrence_resident(const vbg_matrix* m, int adjoint, int* resident);
 
 /* vbg_cheb_step with dots, for callers that cannot let the library allocate
  * device memory (no counterpart in the reference).  vbg_cheb_step allocates

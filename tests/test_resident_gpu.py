@@ -141,3 +141,80 @@ def test_matrix_that_does_not_fit(dev):
         finally:
             _capi.set_option("apply.vec_kernel", 0)
     assert np.abs(outs[0] - outs[1]).max() < 1e-12 * np.abs(outs[1]).max()
+
+
+def _series(dm, v, cf):
+    import torch
+
+    from vbcsr_b200 import _capi
+
+    out = torch.empty_like(v)
+    _capi.call("vbg_cheb_series", dm.h, 1, 1, _ptr(v), len(cf), cf.ctypes.data_as(C.c_void_p), 1.0, 0.0, _ptr(out), 0,
+               None, None)
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+@pytest.mark.parametrize("name", ["lattice", "one_row", "real", "random"])
+@pytest.mark.parametrize("adjoint", [False, True])
+def test_resident_once_the_steps_repay_the_plan(oracle, dev, name, adjoint):
+    """Recurrences of seven steps run step by step until the matrix has run
+    enough of them, then as one launch, in the direction asked for, with the
+    same results."""
+    import torch
+
+    from vbcsr_b200 import _capi
+
+    from . import _gpu
+
+    H = _matrix(name)
+    rng = np.random.default_rng(5)
+    x = _vec(H, rng)
+    dm = _gpu.dmat(H)
+    xd = torch.from_numpy(x).cuda()
+    steps = 7
+    coef = np.ascontiguousarray(np.tile([1.9, -0.1, -1.0, 0.0, 0.0], (steps, 1)))
+    p, y = np.zeros_like(x), x
+    for _ in range(steps):
+        p, y = y, 1.9 * oracle.apply(H, y, adjoint) - 0.1 * y - p
+    calls = 0
+    while not _capi.recurrence_resident(dm, adjoint):
+        assert calls * steps < 12 + H.nnzb // 1500 + steps, "never resident"
+        last = torch.empty_like(xd)
+        _capi.call("vbg_cheb_columns", dm.h, int(adjoint), _ptr(xd), None, steps, coef.ctypes.data_as(C.c_void_p), None,
+                   None, 0, 0, 0, 0, _ptr(last), None, None)
+        torch.cuda.synchronize()
+        assert np.abs(last.cpu().numpy() - y).max() < 1e-11 * np.abs(y).max()
+        calls += 1
+    assert calls > 1
+    assert not _capi.recurrence_resident(dm, not adjoint)
+
+
+def test_long_series_is_resident_at_once(dev):
+    import torch
+
+    from vbcsr_b200 import _capi
+
+    from . import _gpu
+
+    dm = _gpu.dmat(_matrix("lattice"))
+    v = torch.from_numpy(_vec(_matrix("lattice"), np.random.default_rng(1))).cuda()
+    _series(dm, v, np.ones((9, 2)))
+    assert not _capi.recurrence_resident(dm)
+    _series(dm, v, np.ones((64, 2)))
+    assert _capi.recurrence_resident(dm)
+
+
+def test_matrix_that_does_not_fit_is_never_resident(dev):
+    import torch
+
+    from vbcsr_b200 import _capi
+
+    from . import _gpu
+
+    H = W.tmd_lattice(68, seed=9, bond_phase=True)[0]
+    dm = _gpu.dmat(H)
+    v = torch.from_numpy(_vec(H, np.random.default_rng(1))).cuda()
+    for _ in range(2):
+        _series(dm, v, np.ones((256, 2)))
+    assert not _capi.recurrence_resident(dm) and not _capi.recurrence_resident(dm, True)

@@ -82,6 +82,7 @@ _SIGNATURES = {
     "vbg_sddmm": ([_vp, _i, _i, _vp, _vp, _d, _d, _vp, _vp], _i),
     "vbg_cheb_series": ([_vp, _i, _i, _vp, _i, _vp, _d, _d, _vp, _i, _vp, _vp], _i),
     "vbg_cheb_columns": ([_vp, _i, _vp, _vp, _i, _vp, _vp, _vp, C.c_int64, _i, _i, _i, _vp, _vp, _vp], _i),
+    "vbg_recurrence_resident": ([_vp, _i, _pi], _i),
     "vbg_apply_tile_rows": ([_vp, _i, _i, _pi], _i),
     "vbg_matrix_create_device": ([C.POINTER(_vp), _i, _i, _vp, C.c_int64, _vp, _vp, _vp, _vp], _i),
     "vbg_square_polynomial_upper": ([_vp, _d, _d, _d, _d, _d, _d, _d, C.POINTER(_vp), _vp], _i),
@@ -158,6 +159,13 @@ def adjoint_kernel(dm: "DeviceMatrix", ld: int) -> str:
     out = C.c_int(-1)
     call("vbg_adjoint_kernel", dm.h, int(ld), C.byref(out))
     return KERNEL_NAMES[out.value]
+
+
+def recurrence_resident(dm: "DeviceMatrix", adjoint: bool = False) -> bool:
+    """Whether vector recurrences on this matrix have run as one launch."""
+    out = C.c_int(0)
+    call("vbg_recurrence_resident", dm.h, int(bool(adjoint)), C.byref(out))
+    return bool(out.value)
 
 
 def apply_tile_rows(dm: "DeviceMatrix", ld: int, precision: int = 0) -> int:

@@ -2431,6 +2431,13 @@ int vbg_cheb_columns(const vbg_matrix* m, int adjoint, const void* x0, const voi
   return p ? copy(before, p) : 0;
 }
 
+int vbg_recurrence_resident(const vbg_matrix* m, int adjoint, int* resident) {
+  VBG_CHECK(m && resident, VBG_E_ARG, "null argument");
+  const auto& plan = m->resident[adjoint ? 1 : 0];
+  *resident = plan && plan->ran ? 1 : 0;
+  return 0;
+}
+
 int vbg_kpm_moments(const vbg_matrix* m, int R, int ld, const void* V0, int M, int precision, int two_moment,
                     int use_graph, double* moments, void* stream) {
   VBG_CHECK(m && V0 && moments, VBG_E_ARG, "null argument");

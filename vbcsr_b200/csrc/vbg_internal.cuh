@@ -227,7 +227,9 @@ struct ChainPlan {
 struct ResidentPlan {
   int grid = 0;
   size_t smem = 0;
-  DevBuf cta, rows, xlist, place;
+  bool ran = false;    // a recurrence has run on it
+  DevBuf data;         // CTA records, row records, X lists, places
+  size_t off[4] = {};  // where each begins
 };
 
 // CUDA-graph cache entry for a replayable recurrence.
@@ -319,6 +321,7 @@ struct vbg_matrix {
   std::map<std::pair<int, int>, std::unique_ptr<vbg::ChainPlan>> chain_plans;
   // Resident vector recurrences, [0] over the rows, [1] over the columns.
   std::unique_ptr<vbg::ResidentPlan> resident[2];
+  int64_t recur_steps = 0;  // vector recurrence steps this structure has run
   // The autotuner's choice of forward multivector kernel (VBG_KERNEL_*) per
   // (leading dimension, FP32 values).
   std::map<std::pair<int, int>, int> tuned;
@@ -356,6 +359,7 @@ struct vbg_matrix {
     chain_plans.clear();
     resident[0].reset();
     resident[1].reset();
+    recur_steps = 0;
     tuned.clear();
     invalidate_values();
   }

@@ -35,6 +35,12 @@ constexpr int kResThreads = 512;
 constexpr size_t kResSmemMax = 226 * 1024;
 constexpr int kResMinSteps = 4;   // fewer steps do not repay the copy of the values
 constexpr int kResRowsPerCta = 8; // fewest block rows a CTA is used for
+// A plan costs the host about 60 us and 3.5 ns a block, a resident step saves 3 to
+// 6 us: it is made when a matrix has run this many steps of recurrences and one
+// more for every so many blocks (made at once, the first series of 5 terms on a
+// 60 x 60 lattice took 1.1 ms instead of 0.27).
+constexpr int kResPlanSteps = 12;
+constexpr int kResPlanBlocks = 1500;
 
 // Per step {alpha, beta, gamma, re c, im c}.
 constexpr int kResCoef = 5;
@@ -307,43 +313,47 @@ static int resident_plan(const vbg_matrix* cm, bool adj, cudaStream_t s, Residen
   const int ctas = std::max(1, std::min(sms, n / kResRowsPerCta));
   std::vector<int4> h_cta(2 * (size_t)ctas), h_rows(2 * (size_t)n);
   std::vector<int> h_x, where(n, -1), stamp(n, -1);
-  std::vector<unsigned short> h_place;
-  std::vector<int64_t> kof(n, 0);
+  int64_t places = 0;  // scalar columns over all rows
+  for (const int j : *src) places += bsz[j];
+  std::vector<unsigned short> h_place(places);
+  h_x.reserve((size_t)m->N * 4);
   int64_t done = 0;
   size_t smem = 0;
-  bool fits = true;
-  int row = 0;
+  bool fits = places < (int64_t)INT32_MAX;
+  int row = 0, p_at = 0;
   for (int b = 0; b < ctas && fits; ++b) {
     const int first = row;
-    const int x_first = (int)h_x.size(), p_first = (int)h_place.size();
+    const int x_first = (int)h_x.size(), p_first = p_at;
     int64_t nv = 0;
-    auto use = [&](int j) {  // X elements of block j in this CTA's list
-      if (stamp[j] == b) return;
-      stamp[j] = b;
-      where[j] = (int)h_x.size() - x_first;
-      for (int q = 0; q < bsz[j]; ++q) h_x.push_back((int)(m->h_scal_off[j] + q));
+    auto use = [&](int j) {  // place of block j's X elements in this CTA's list
+      if (stamp[j] != b) {
+        stamp[j] = b;
+        where[j] = (int)h_x.size() - x_first;
+        const int x0 = (int)m->h_scal_off[j];
+        for (int q = 0; q < bsz[j]; ++q) h_x.push_back(x0 + q);
+      }
+      return where[j];
     };
     // rows until this CTA's share of the values is reached (the last takes
     // the rest), leaving a row for each CTA to come
     while (row < n && (b + 1 == ctas || ((done * ctas < (int64_t)(b + 1) * m->nnz || row == first) &&
                                          n - row > ctas - 1 - b))) {
-      int64_t K = 0;
-      use(row);
-      const int p_row = (int)h_place.size() - p_first;
+      const int own = use(row), p_row = p_at - p_first;
+      unsigned short* pp = h_place.data() + p_at;
       for (int e = (*ptr)[row]; e < (*ptr)[row + 1]; ++e) {
-        const int j = (*src)[e];
-        use(j);
-        for (int q = 0; q < bsz[j]; ++q) h_place.push_back((unsigned short)(where[j] + q));
-        K += bsz[j];
+        const int j = (*src)[e], w0 = use(j), w1 = w0 + bsz[j];
+        for (int w = w0; w < w1; ++w) *pp++ = (unsigned short)w;
       }
+      const int64_t K = pp - (h_place.data() + p_at);
+      p_at += (int)K;
       h_rows[2 * (size_t)row] = make_int4((int)nv, (int)K, p_row, bsz[row]);
-      h_rows[2 * (size_t)row + 1] = make_int4(where[row], (int)m->h_scal_off[row], 0, 0);
+      h_rows[2 * (size_t)row + 1] = make_int4(own, (int)m->h_scal_off[row], 0, 0);
       nv += K * bsz[row];
       done += K * bsz[row];
       ++row;
       if (nv * (int64_t)es > (int64_t)kResSmemMax) break;
     }
-    const int nx = (int)h_x.size() - x_first, np = (int)h_place.size() - p_first;
+    const int nx = (int)h_x.size() - x_first, np = p_at - p_first;
     h_cta[2 * (size_t)b] = make_int4(first, row, x_first, nx);
     h_cta[2 * (size_t)b + 1] = make_int4((int)nv, np, p_first, 0);
     const size_t bytes = res_smem(nv, nx, np, row - first, es);
@@ -351,16 +361,22 @@ static int resident_plan(const vbg_matrix* cm, bool adj, cudaStream_t s, Residen
     fits = bytes <= kResSmemMax && nx <= 65535;
   }
   if (fits && row == n) {
-    plan->smem = smem;
-    if ((rc = plan->cta.ensure(h_cta.size() * sizeof(int4), s))) return rc;
-    if ((rc = plan->rows.ensure(h_rows.size() * sizeof(int4), s))) return rc;
-    if ((rc = plan->xlist.ensure(std::max<size_t>(h_x.size(), 1) * sizeof(int), s))) return rc;
-    if ((rc = plan->place.ensure(std::max<size_t>(h_place.size(), 1) * 2, s))) return rc;
-    VBG_CUDA(cudaMemcpyAsync(plan->cta.p, h_cta.data(), h_cta.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
-    VBG_CUDA(cudaMemcpyAsync(plan->rows.p, h_rows.data(), h_rows.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
-    VBG_CUDA(cudaMemcpyAsync(plan->xlist.p, h_x.data(), h_x.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-    VBG_CUDA(cudaMemcpyAsync(plan->place.p, h_place.data(), h_place.size() * 2, cudaMemcpyHostToDevice, s));
+    // one buffer, one copy
+    const size_t sizes[4] = {h_cta.size() * sizeof(int4), h_rows.size() * sizeof(int4), h_x.size() * sizeof(int),
+                             h_place.size() * sizeof(unsigned short)};
+    const void* parts[4] = {h_cta.data(), h_rows.data(), h_x.data(), h_place.data()};
+    size_t total = 0;
+    for (int k = 0; k < 4; ++k) {
+      plan->off[k] = total;
+      total += (sizes[k] + 15) / 16 * 16;
+    }
+    std::vector<char> stage(total);
+    for (int k = 0; k < 4; ++k)
+      if (sizes[k]) std::memcpy(stage.data() + plan->off[k], parts[k], sizes[k]);
+    if ((rc = plan->data.ensure(total, s))) return rc;
+    VBG_CUDA(cudaMemcpyAsync(plan->data.p, stage.data(), total, cudaMemcpyHostToDevice, s));
     VBG_CUDA(cudaStreamSynchronize(s));  // the host vectors are locals
+    plan->smem = smem;
     plan->grid = ctas;
     *out = plan.get();
   }
@@ -369,7 +385,7 @@ static int resident_plan(const vbg_matrix* cm, bool adj, cudaStream_t s, Residen
 }
 
 template <typename T, bool ADJ>
-static int launch_resident_t(ResidentArgs& a, const ResidentPlan* plan, const T* vals, cudaStream_t s, bool* ran) {
+static int launch_resident_t(ResidentArgs& a, ResidentPlan* plan, const T* vals, cudaStream_t s, bool* ran) {
   static int state[kMaxDevices] = {};  // 1: usable, 2: not
   const int dev = current_device();
   if (!state[dev]) {
@@ -385,6 +401,7 @@ static int launch_resident_t(ResidentArgs& a, const ResidentPlan* plan, const T*
   void* params[2] = {&a, &vals};
   VBG_CUDA(cudaLaunchCooperativeKernel((const void*)resident_kernel<T, ADJ>, dim3(plan->grid), dim3(kResThreads),
                                        params, plan->smem, s));
+  plan->ran = true;
   return 0;
 }
 
@@ -398,6 +415,10 @@ static int resident_run(const vbg_matrix* m, bool adj, ResidentArgs& a, const do
   if (a.steps < kResMinSteps || m->N == 0 || m->max_bs > 8) return 0;
   cudaStreamCaptureStatus st;
   if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return 0;
+  // the plan once the matrix's recurrences, this one among them, repay it
+  auto* mm = const_cast<vbg_matrix*>(m);
+  mm->recur_steps += a.steps;
+  if (!m->resident[adj ? 1 : 0] && mm->recur_steps < kResPlanSteps + m->nnzb / kResPlanBlocks) return 0;
   ResidentPlan* plan = nullptr;
   int rc = resident_plan(m, adj, s, &plan);
   if (rc || !plan) return rc;
@@ -412,10 +433,11 @@ static int resident_run(const vbg_matrix* m, bool adj, ResidentArgs& a, const do
   a.xch[1] = static_cast<char*>(a.xch[0]) + vec;
   VBG_CUDA(cudaMemsetAsync(base, 0, 256, s));
   VBG_CUDA(cudaMemcpyAsync(base + 256, coef, cb, cudaMemcpyHostToDevice, s));
-  a.cta = plan->cta.as<int4>();
-  a.rows = plan->rows.as<int4>();
-  a.xlist = plan->xlist.as<int>();
-  a.place = plan->place.as<unsigned short>();
+  const char* pd = plan->data.as<char>();
+  a.cta = reinterpret_cast<const int4*>(pd + plan->off[0]);
+  a.rows = reinterpret_cast<const int4*>(pd + plan->off[1]);
+  a.xlist = reinterpret_cast<const int*>(pd + plan->off[2]);
+  a.place = reinterpret_cast<const unsigned short*>(pd + plan->off[3]);
   a.ptr = (adj ? m->csc_ptr : m->row_ptr).as<int>();
   a.ent_slot = adj ? m->csc_slot.as<int>() : nullptr;
   a.ent_src = (adj ? m->csc_row : m->col_ind).as<int>();
