@@ -133,16 +133,18 @@ __global__ void __launch_bounds__(kSddmmWarps * 32, 4)
 // columns: a row's G operands stay in registers, and the X operands and old
 // output values of several blocks are loaded before their products -- the
 // general form waits for each block's rows, then for its output.
-constexpr int kSddmmFrags = 4;  // 16-byte operands per lane
+// F: 16-byte operands per lane.  At one operand (8 real, 4 complex columns) four
+// CTAs share an SM instead of two.
+constexpr int kSddmmFrags = 4;
 
-template <typename T, bool V2>
-__global__ void __launch_bounds__(kSddmmWarps * 32, 2)
+template <typename T, bool V2, int F>
+__global__ void __launch_bounds__(kSddmmWarps * 32, F == 1 ? 4 : 2)
     sddmm_small_kernel(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ col_ind,
                        const int* __restrict__ bsz, const int64_t* __restrict__ scal_off,
                        const int64_t* __restrict__ blk_off, int k, int ld, const T* __restrict__ G,
                        const T* __restrict__ X, double are, double aim, int split, T* __restrict__ out) {
   constexpr bool CX = std::is_same<T, cplx>::value;
-  constexpr int F = kSddmmFrags, KF = CX ? 4 : 8;  // columns per operand
+  constexpr int KF = CX ? 4 : 8;                   // columns per operand
   constexpr int B = CX ? 2 : 3;                     // blocks in flight
   const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const T alpha = scalar_from<T>(are, aim);
@@ -239,14 +241,29 @@ __global__ void __launch_bounds__(kSddmmWarps * 32, 2)
 template <typename T, bool V2>
 static int launch_sddmm(const vbg_matrix* m, int k, int ld, const void* G, const void* X, double are, double aim,
                         void* out, cudaStream_t s) {
-  // several tasks per resident warp, so that the last ones end together
+  const int kf = std::is_same<T, cplx>::value ? 4 : 8;
+  const bool small = m->max_bs <= 8 && k <= kSddmmFrags * kf, one = small && k <= kf;
   int split = 1;
-  while (split < 4 && (int64_t)m->n * split < (int64_t)sm_count() * 128 && m->nnzb >= 4 * (int64_t)split * m->n)
-    split *= 2;
+  if (small) {
+    // a row's blocks go to several warps while all are resident at once; two
+    // when the rows make one to four rounds of them, so that the last round
+    // ends together (us, split 1 / 2 / 4, blocks of 2-4, 32 columns: 500 rows 14
+    // / 9 / 8, 1000 of 4-8 15 / 11 / 13, 2000 15 / 17 / 19, 5000 35 / 33 / 37,
+    // 12000 64 / 64 / 78)
+    const int64_t wave = (int64_t)sm_count() * 16;
+    if (m->n <= wave) {
+      while (split < 4 && 2 * (int64_t)m->n * split <= wave && m->nnzb >= 4 * (int64_t)split * m->n) split *= 2;
+    } else if (m->n < 4 * wave && m->nnzb >= 4 * (int64_t)m->n) {
+      split = 2;
+    }
+  } else {
+    // several tasks per resident warp, so that the last ones end together
+    while (split < 4 && (int64_t)m->n * split < (int64_t)sm_count() * 128 && m->nnzb >= 4 * (int64_t)split * m->n)
+      split *= 2;
+  }
   const int64_t want = ((int64_t)m->n * split + kSddmmWarps - 1) / kSddmmWarps;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sm_count() * 8));
-  const int kmax = kSddmmFrags * (std::is_same<T, cplx>::value ? 4 : 8);
-  auto* kernel = m->max_bs <= 8 && k <= kmax ? sddmm_small_kernel<T, V2> : sddmm_kernel<T, V2>;
+  auto* kernel = one ? sddmm_small_kernel<T, V2, 1> : small ? sddmm_small_kernel<T, V2, kSddmmFrags> : sddmm_kernel<T, V2>;
   kernel<<<grid, kSddmmWarps * 32, 0, s>>>(
       m->n, m->row_ptr.as<int>(), m->col_ind.as<int>(), m->bsz.as<int>(), m->scal_off.as<int64_t>(),
       m->blk_off.as<int64_t>(), k, ld, static_cast<const T*>(G), static_cast<const T*>(X), are, aim, split,
