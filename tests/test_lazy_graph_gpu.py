@@ -54,3 +54,25 @@ def test_duplicates_and_values(pair, dev):
     T = A.transpose()
     assert np.array_equal(T.to_dense(), H.to_dense().T)
     assert T.get_block(0, 0).shape == (H.block_sizes[0], H.block_sizes[0])
+
+
+@pytest.mark.parametrize("n", [60, 2500])  # below and above the megabyte that get_values keeps
+def test_values_again_after_changes(n, dev):
+    from vbcsr_b200 import VBCSR
+
+    H = W.banded_decaying(n, neighbours=4, band=8, seed=3)
+    assert (H.nnz * 8 > 1 << 20) == (n == 2500)
+    A = VBCSR.from_block_csr(H.block_sizes, H.row_ptr, H.col_ind, H.values)
+    A.scale(2.0)
+    first = A.get_values()
+    assert np.array_equal(first, 2.0 * H.values) and np.array_equal(A.get_values(), first)
+    first[:] = 0.0  # the caller's own array
+    assert np.array_equal(A.get_values(), 2.0 * H.values)
+    A.scale(0.5)
+    assert np.array_equal(A.get_values(), H.values)
+    assert np.array_equal(A.get_block(1, 1).ravel(), H.values[H.slot_offsets()[H.row_ptr[1] + list(
+        H.col_ind[H.row_ptr[1]:H.row_ptr[2]]).index(1)]:][:A.get_block(1, 1).size])
+    A.fill(3.0)
+    assert np.all(A.get_values() == 3.0)
+    A.scale(2.0)
+    assert np.all(A.get_values() == 6.0)

@@ -709,9 +709,12 @@ void bind_matrix(py::module& m, const char* name) {
         return out;
       }, py::arg("row"), py::arg("col"))
       .def("get_values", [](M& a) {
+        // up to 1 MB through the host copy, which later calls then read (17 us for
+        // 0.2 MB instead of a transfer's 59); more straight into the result (filling
+        // the copy first took 84 ms for 144 MB, and from then on saved little: 88
+        // MB again 68 ms from the copy, 73 from the device)
+        if (!a.host_ok && a.nnz() * sizeof(T) <= (1u << 20)) a.ensure_host();
         if (a.host_ok) return to_array(a.host);
-        // straight into the result (the host copy is left for those who
-        // change it: filling it first and copying it took 84 ms for 144 MB)
         py::array_t<T> out((py::ssize_t)a.nnz());
         if (out.size()) check(vbg_matrix_get_values(a.dm, out.mutable_data(), stream()), "vbg_matrix_get_values");
         return out;

@@ -570,6 +570,9 @@ class VBCSR(LinearOperator):
         return np.asarray(self._core.col_ind, dtype=np.int32)
 
     def get_values(self) -> np.ndarray:
+        """The stored values in slot order.  Values last changed on the device are
+        copied from there; over 1 MB by every call, so a program that reads
+        them several times keeps the array."""
         return np.asarray(self._core.get_values(), dtype=self.dtype)
 
     def save_matrix_market(self, filename) -> None:
