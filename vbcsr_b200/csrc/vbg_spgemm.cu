@@ -948,7 +948,8 @@ static int spgemm_run(const vbg_matrix* A, const vbg_matrix* B, double thr, int 
   // its bound (sym_need_kernel) allows, in one temporary list, so that one pass counts
   // and writes them (a second pass over the pairs cost as much again: 190 of
   // 325 us on 12000 rows of 29 blocks).  Products whose bounds add up to more
-  // than kSymTempMax columns count first and write in a second pass.
+  // than kSymTempMax columns, or to more than there is memory for beside the
+  // tables, count first and write in a second pass.
   std::vector<int> sym_rows;
   std::vector<int64_t> sym_off;
   int64_t sym_room = 0;
@@ -958,16 +959,21 @@ static int spgemm_run(const vbg_matrix* A, const vbg_matrix* B, double thr, int 
       sym_off.push_back(sym_room);
       sym_room += need[i] >> 32;
     }
-  const bool one_pass = sym_room <= kSymTempMax;
+  bool one_pass = sym_room <= kSymTempMax;
   DevBuf sym_tmp(s), sym_off_dev(s);
   if ((rc = rows_dev.ensure(std::max<size_t>(sym_rows.size(), 1) * sizeof(int)))) return rc;
   if (!sym_rows.empty())
     VBG_CUDA(cudaMemcpyAsync(rows_dev.p, sym_rows.data(), sym_rows.size() * sizeof(int), cudaMemcpyHostToDevice, s));
   if (one_pass && !sym_rows.empty()) {
-    if ((rc = sym_tmp.ensure(std::max<int64_t>(sym_room, 1) * sizeof(int)))) return rc;
-    if ((rc = sym_off_dev.ensure(sym_off.size() * sizeof(int64_t)))) return rc;
-    VBG_CUDA(cudaMemcpyAsync(sym_off_dev.p, sym_off.data(), sym_off.size() * sizeof(int64_t), cudaMemcpyHostToDevice,
-                             s));
+    if (!(rc = sym_tmp.ensure(std::max<int64_t>(sym_room, 1) * sizeof(int))))
+      rc = sym_off_dev.ensure(sym_off.size() * sizeof(int64_t));
+    if (rc && rc != VBG_E_NOMEM) return rc;
+    one_pass = !rc;
+    if (one_pass)
+      VBG_CUDA(cudaMemcpyAsync(sym_off_dev.p, sym_off.data(), sym_off.size() * sizeof(int64_t), cudaMemcpyHostToDevice,
+                               s));
+    else
+      sym_tmp.release();
   }
   SymArgs sa{};
   sa.a_rp = A->row_ptr.as<int>();
@@ -1006,7 +1012,13 @@ static int spgemm_run(const vbg_matrix* A, const vbg_matrix* B, double thr, int 
                            return 0;
                          });
   };
-  if ((rc = sym_launch(1, one_pass ? 1 : 0, nullptr, sym_tmp.as<int>(), sym_off_dev.as<int64_t>()))) return rc;
+  rc = sym_launch(1, one_pass ? 1 : 0, nullptr, sym_tmp.as<int>(), sym_off_dev.as<int64_t>());
+  if (rc == VBG_E_NOMEM && one_pass) {  // no room for the tables beside the list
+    one_pass = false;
+    sym_tmp.release();
+    rc = sym_launch(1, 0, nullptr, nullptr, nullptr);
+  }
+  if (rc) return rc;
   // C's row pointers: exclusive scan of the per-row counts on the device
   DevBuf d_crp(s), d_cci(s), scan_tmp(s);
   if ((rc = d_crp.ensure((n + 1) * sizeof(int)))) return rc;
@@ -1039,6 +1051,7 @@ static int spgemm_run(const vbg_matrix* A, const vbg_matrix* B, double thr, int 
     gather_columns_kernel<<<std::max(1, std::min((nr + 7) / 8, sm_count() * 16)), 256, 0, s>>>(
         nr, rows_dev.as<int>(), sym_off_dev.as<int64_t>(), sym_tmp.as<int>(), d_crp.as<int>(), d_cci.as<int>());
     VBG_CUDA(cudaGetLastError());
+    sym_tmp.release();  // before the values: up to 1 GB
   }
   int herr[4] = {0, 0, 0, 0};
   VBG_CUDA(cudaMemcpyAsync(herr, err.p, 16, cudaMemcpyDeviceToHost, s));
