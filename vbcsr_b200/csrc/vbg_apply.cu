@@ -1447,8 +1447,9 @@ static int prepare(const vbg_matrix* m, bool adj, int k, int ld, ApplyArgs& a, c
 // apply takes).  A tensor-core step holds 32 values however few a block fills,
 // while a warp here spends its lanes on columns and its lane groups on several
 // blocks, but the block sizes' launches follow one another.  So: blocks of at
-// most 7 values on average, with at least 1200 block rows a size, unless the
-// columns leave over a quarter of the lanes idle (nvec 16-byte vectors a row;
+// most 7 values on average, with at least 1200 block rows a size (3600 where
+// real columns leave lanes idle: 5000 rows of 1-2, 96 columns 57 / 65, 20000 of
+// 1-2 161 / 127), unless the columns leave over a quarter of the lanes idle (nvec 16-byte vectors a row;
 // lane groups need a power of two below 32) and the blocks are not single
 // values (20000 rows, real 24 columns: sizes 1-2 68 / 66, 1 66 / 50).  And complex adjoints of larger small blocks,
 // whose steps are four real ones, on many rows: whole warps of columns, or so
@@ -1469,7 +1470,9 @@ static bool lane_rows(const vbg_matrix* m, const ApplyArgs& a, bool adj) {
   const int nvec = a.ld / VT<T>::E;
   const bool lanes = nvec < 24 ? (nvec & (nvec - 1)) == 0 : 4 * nvec >= 3 * ((nvec + 31) / 32 * 32);
   const double mean = (double)m->nnz / (double)m->nnzb;
-  if (mean <= (lanes ? 7.0 : 1.5) && m->n >= 1200 * (int64_t)m->class_segs.size()) return true;
+  const bool full = nvec < 32 ? (nvec & (nvec - 1)) == 0 : nvec % 32 == 0;
+  const int64_t rows = (cx || full ? 1200 : 3600) * (int64_t)m->class_segs.size();
+  if (mean <= (lanes ? 7.0 : 1.5) && m->n >= rows) return true;
   return cx && adj && mean <= 15.0 && m->n >= 8000 && (nvec <= 4 || nvec == 24 || nvec % 32 == 0);
 }
 
@@ -1520,14 +1523,13 @@ static int launch_fwd_mv(const vbg_matrix* m, const ApplyArgs& a, const T* v, cu
 // applies.  FP64 and
 // complex: rows (lane_rows or on the tensor cores), except where the pipelined
 // kernel, whose cost goes with the values, is faster.  On rows of a multiple of
-// 512 bytes it fills whole warps: blocks of at most 20 values on average, or
-// many real rows of one block size at 512 bytes, once there are rows enough to
-// fill the SMs with its warps of 512 bytes (3000; complex, whose products are
-// four times the work, 2500).  On other complex rows: blocks of at most 10
+// 512 bytes it fills whole warps: blocks of at most 20 values on average, once
+// there are rows enough to fill the SMs with its warps of 512 bytes (3000;
+// complex, whose products are four times the work, 2500).  On other complex rows: blocks of at most 10
 // values, whose products would be four tensor-core steps each.
 // us an apply, pipelined / tensor-core rows, random rows of 13 blocks, real 64
 // columns: 20000 rows of sizes 2-4 (mean 9) 99 / 130, 3-5 (16) 109 / 151, 4-8
-// (36) 412 / 169, 8 (64) 175 / 195; 5000 rows 2-4 36 / 38, 3-5 40 / 40, 8
+// (36) 412 / 169, 8 (64) 175 / 195 (but a Chebyshev step with its dots 233 / 211); 5000 rows 2-4 36 / 38, 3-5 40 / 40, 8
 // 62 / 54; 1500 rows 2-4 32 / 19; 500 rows 2-4 32 / 11, where tiles of 4 rows
 // took 13.  Real 128 columns, 20000 rows: 203 / 287, 229 / 311, 560 / 351, 8
 // 369 / 345; complex 16 columns 1-2 (2) 77 / 106, 2-4 99 / 107, 3-5 120 / 116,
@@ -1543,7 +1545,7 @@ static int untiled_choice(const vbg_matrix* m, const ApplyArgs& a, cudaStream_t 
   bool pipe = f32;
   if (!f32 && bytes % 512 == 0) {
     const bool enough = m->n * (bytes / 512) >= (cx ? 2500 : 3000);
-    pipe = enough && (mean <= 20.0 || (!cx && bytes == 512 && m->min_bs == m->max_bs && m->n >= 16000));
+    pipe = enough && mean <= 20.0;
   } else if (cx) {
     pipe = mean <= 10.0;
   }
