@@ -77,8 +77,8 @@ int vbg_device_status(unsigned* status, int clear);
  *                  given leading dimension and precision on a matrix (outside
  *                  stream capture; vbg_kpm_moments* before their capture)
  *                  chooses its kernel: by the structure and sizes where
- *                  kernels add in different orders, by timing between the
- *                  ones that add alike (tiles and chained tiles at 512-byte
+ *                  kernels add a row in different orders, by timing between
+ *                  the ones that add it alike (tiles and chained tiles at 512-byte
  *                  rows, FP32 at 64 columns and up); the trials overwrite Y
  *                  and the dots, never the accumulator.
  *                  0: the default order (chained tiles for FP32 only).

@@ -1195,10 +1195,11 @@ static bool tile_queue_on(const vbg_matrix* m, int ld, int es) {
 }
 
 // Pieces of 128 bytes of a multivector row with leading dimension ld that
-// apply_dtile_kernel<T, NP> takes (1 or 2), else 0.  At four pieces the
-// tensor pipe (blocks of 3 and 5 fill 3 and 5 eighths of a step) is the
-// bound, and scalar multiply-adds with two columns a lane are faster: 200 x
-// 200 lattice, FP64, 64 columns: 410 us a step against 313.
+// apply_dtile_kernel<T, NP> takes (1 or 2), else 0.  At four pieces scalar
+// multiply-adds with two columns a lane are faster (200 x 200 lattice, FP64, 64
+// columns: 410 us a step against 313).  Not for the tensor pipe, which the
+// padded steps of blocks of 3 and 5 kept 37 % busy; what else held that form
+// back (129 M warp instructions at 16 warps an SM) was not pursued.
 template <typename T>
 static int dtile_pieces(int ld) {
   const int64_t bytes = (int64_t)ld * (int)sizeof(T);
@@ -1585,8 +1586,9 @@ static int autotune_fwd(const vbg_matrix* m, const ApplyArgs& a0, const T* v, cu
   auto* mm = const_cast<vbg_matrix*>(m);
   const auto cap_key = std::make_pair(a.ld, (int)sizeof(T));
   // Kernels that add a row's products in different orders are not timed
-  // against each other, so that equal matrices give equal bits whatever the
-  // clock said.  FP64 and complex values at 512-byte rows: tiles, chained or
+  // against each other, so that equal matrices give the same bits in Y whatever
+  // the clock said.  (The dots may differ in their last bits: tile height and
+  // order, which are timed, decide whose partial sums a CTA holds.)  FP64 and complex values at 512-byte rows: tiles, chained or
   // not (which add alike), where tiles of at least 8 block rows fit, else
   // untiled_choice.  FP32 at 64 columns and up: as timed (the chained, tiled
   // and pipelined forms add alike).
@@ -1702,7 +1704,8 @@ static int fwd_choice(const vbg_matrix* m, bool f32, const ApplyArgs& a, const T
 // scalar-row kernel (VBG_KERNEL_SCALAR_ROWS; *srow_out set).  Option
 // "apply.vec_kernel" forces one; at 0 the autotuner times both on the first
 // vector apply per matrix and precision (three launches each, the
-// accumulator off) and keeps the faster.  Untuned (autotuner off, no
+// accumulator off) and keeps the faster (they add in different orders: where
+// they are about as fast, the last bits of a vector depend on the clock).  Untuned (autotuner off, no
 // allocation allowed, or the stream being captured) complex values take the
 // scalar-row kernel, real ones a warp per block row.
 template <typename T, bool ADJ = false>

@@ -18,9 +18,12 @@
 // What bounds it: B's fragments from L2 (each serves both rows) and the
 // instructions around the tensor steps.  One C block per warp and pass, as it
 // was before, loaded both fragments for every pair, kept a list entry with
-// two 64-bit offsets per pair, and ran one launch per block size in series:
-// 52 instructions a pair (now about 10).  12000 rows of 4-8, 29 blocks a row,
-// 8.3 M pairs: 1.93 ms before.
+// two 64-bit offsets per pair, and ran one launch per block size in series (52
+// instructions a pair, 1.93 ms on 12000 rows of 4-8, 29 blocks a row, 8.3 M
+// pairs).  Warp instructions a kept pair now: 34 in the dense form (3000 rows of
+// 121 full blocks of 6, 43 M pairs: 2.67 ms, tensor pipe active 45 %), 82 in the
+// sparse form on the 8.3 M pairs (1.38 ms, 17 %), whose short lists pay for the
+// walk of B's columns.
 #include <algorithm>
 #include <type_traits>
 
@@ -489,8 +492,13 @@ static int launch_pairs(const PairsArgs& a, bool gated, bool dense, int warps, s
 
 // The share of C's blocks' inner columns that hold a pair from which a pass
 // over all of them with J products each (DENSE) beats running through every
-// C column's own pairs: about 8 instructions a product when all are there but
-// 96 at a quarter, against 20.
+// C column's own pairs.  Whole products, us, dense / sparse form, blocks of 4-8:
+// share 0.26 (31 of 65 columns of a band) 1716 / 1333, complex 2502 / 2206; 0.33
+// 2170 / 1736 and 3414 / 3621; 0.41 1004 / 888 and 1563 / 1680; random rows of
+// 160 blocks at 0.5 682 / 663 and 705 / 940, at 0.7 714 / 911 and 983 / 1388.
+// Full bands of blocks of 6 (share 0.5): 65 blocks a row 1376 / 1247, 121 3238 /
+// 3503, 201 8421 / 14374; complex 49 1579 / 1503, 65 2460 / 2594, 121 7191 /
+// 10827: the longer the rows, the fewer CTAs of the sparse form share an SM.
 constexpr double kDenseShare = 0.45;
 
 int numeric_pairs(const vbg_matrix* A, const vbg_matrix* B, vbg_matrix* C, const RowPairs& ka, int max_k,

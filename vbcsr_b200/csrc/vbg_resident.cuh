@@ -6,7 +6,7 @@
 // (+ c_s g) of a few hundred steps on a matrix whose values fit the SMs'
 // shared memory (148 x 227 KB) reads the same 30 MB from L2 at every step when
 // each step is a launch of its own, and pays a launch and its tail per step:
-// 14.6 us a step on a 60 x 60 lattice with complex values (28.7 MB).  Here
+// 14.5 us a step on a 60 x 60 lattice with complex values (28.7 MB).  Here
 // one cooperative launch runs all steps: a CTA per SM copies the values of
 // its block rows into shared memory once (as r x K panels, K the scalar
 // columns of the row's blocks side by side), and per step gathers the X

@@ -654,7 +654,7 @@ struct Bin {
 // Groups rows by table size.  The bins' launches run one after the other, so
 // a bin too small to fill the SMs joins the next larger one (a few rows at
 // the ends of a band otherwise cost a launch of their own, 25 us for one
-// CTA), unless its tables would grow more than fourfold.
+// CTA), unless the next larger one's tables are over four times its own.
 constexpr size_t kSmallBin = 2048;
 static std::vector<Bin> make_bins(const std::vector<int64_t>& need) {
   std::map<int, std::vector<int>> by;
@@ -678,9 +678,9 @@ static std::vector<Bin> make_bins(const std::vector<int64_t>& need) {
 // column range those B rows cover (their columns are sorted), bounds its
 // columns; the table needs 2 b + 1 entries, or the span where that is less:
 // columns of one span never collide in a table as large.  need[i] = b << 32 |
-// entries; -1 for an empty row; *pairs the sum of those lengths.  `upper`: only columns >= i are inserted, so
-// the span starts at i at the earliest (-1 when every column lies below the
-// row).
+// entries; -1 for an empty row; *pairs the sum of those lengths.  `upper`: only
+// columns >= i are inserted, so the span starts at i at the earliest (-1 when
+// every column lies below the row).
 __global__ void sym_need_kernel(int n, const int* __restrict__ a_rp, const int* __restrict__ a_ci,
                                 const int* __restrict__ b_rp, const int* __restrict__ b_ci, int upper,
                                 int self_cols, int64_t* __restrict__ need,
@@ -945,8 +945,8 @@ static int spgemm_run(const vbg_matrix* A, const vbg_matrix* B, double thr, int 
   }
   auto sym_bins = make_bins(need);
   // the bins' rows, and where each may put its columns: room for as many as
-  // its bound (sym_need_kernel) allows, in one temporary list, so that one pass counts
-  // and writes them (a second pass over the pairs cost as much again: 190 of
+  // its bound (sym_need_kernel) allows, in one temporary list, so that one pass
+  // counts and writes them (a second pass over the pairs cost as much again: 190 of
   // 325 us on 12000 rows of 29 blocks).  Products whose bounds add up to more
   // than kSymTempMax columns, or to more than there is memory for beside the
   // tables, count first and write in a second pass.
