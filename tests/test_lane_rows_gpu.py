@@ -72,6 +72,15 @@ def test_forward(oracle, dev, cplx, k, n, lo, hi):
     assert _step(oracle, H, k, False) == want
 
 
+@pytest.mark.parametrize("cplx,k,adjoint", [(False, 2, False), (False, 4, True), (True, 2, False), (True, 2, True)])
+@pytest.mark.parametrize("n", [7999, 8000])
+def test_rows_of_32_bytes(oracle, dev, cplx, k, adjoint, n):
+    H = W.random_pattern(n, 2, 4, 5, seed=n)
+    if cplx:
+        _phases(H, n)
+    assert _step(oracle, H, k, adjoint) == ("lane_rows" if n == 8000 else "rows")
+
+
 @pytest.mark.parametrize("k,want", [(4, "lane_rows"), (8, "rows"), (24, "lane_rows"), (48, "rows"), (32, "lane_rows"), (64, "lane_rows")])
 def test_complex_adjoint_on_many_rows(oracle, dev, k, want):
     H = _phases(W.tmd_lattice(52, seed=1)[0], 5)  # 8112 block rows of 3 and 5, mean 14.3 values a block

@@ -1454,7 +1454,10 @@ static int prepare(const vbg_matrix* m, bool adj, int k, int ld, ApplyArgs& a, c
 // lane groups need a power of two below 32) and the blocks are not single
 // values (20000 rows, real 24 columns: sizes 1-2 68 / 66, 1 66 / 50).  And complex adjoints of larger small blocks,
 // whose steps are four real ones, on many rows: whole warps of columns, or so
-// few that the groups take several blocks (4 columns), or 24.
+// few that the groups take several blocks (4 columns), or 24.  And rows of at
+// most 32 bytes on blocks of up to 17 values, which fill a quarter of a piece
+// (30000 rows of 3 and 5, real 2 columns 66 / 58, adjoint 68 / 52, 20000 random
+// rows of 3-5 52 / 46 and 58 / 47; but 5000 of 2-4, adjoint at 4, 23 / 31).
 // us an apply, tensor-core rows / these (20000 random block rows of 13 blocks,
 // adjoint): sizes 1-2 real 8 columns 58 / 29, 64 columns 140 / 89, complex 16
 // columns 105 / 55; sizes 2-3 74 real 32 columns / 61; sizes 2-4 (mean 9) real
@@ -1474,6 +1477,7 @@ static bool lane_rows(const vbg_matrix* m, const ApplyArgs& a, bool adj) {
   const bool full = nvec < 32 ? (nvec & (nvec - 1)) == 0 : nvec % 32 == 0;
   const int64_t rows = (cx || full ? 1200 : 3600) * (int64_t)m->class_segs.size();
   if (mean <= (lanes ? 7.0 : 1.5) && m->n >= rows) return true;
+  if (nvec <= 2 && mean <= 17.0 && m->n >= 8000) return true;
   return cx && adj && mean <= 15.0 && m->n >= 8000 && (nvec <= 4 || nvec == 24 || nvec % 32 == 0);
 }
 
